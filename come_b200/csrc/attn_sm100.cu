@@ -1,24 +1,33 @@
 // Variable-length biased attention forward on Blackwell tensor cores (sm_100a): tcgen05.mma with TMEM
 // accumulators, TMA-fed 128-byte-swizzled Q/K/V tiles, warp-specialised roles.
 //
-// Persistent kernel: one CTA per SM walks the work items; a work item is the (up to) three 128-row query tiles of one
+// Persistent kernel: one CTA per SM walks the work items; a work item is one to four 128-row query tiles of one
 // (segment, head), whose keys are walked 64 at a time.  Barrier phases keep counting across items.
-//   warps 0-3 / 4-7 / 8-11 : softmax group of query tile 0 / 1 / 2.  Thread r owns score row r (TMEM lane r).  Per key
-//                     tile it pulls the 64 scores into registers (S is free for the next Q K^T at once), takes the row
-//                     max with 3-input max, then p = exp2(s * scale*log2e - m) in packed float32x2 arithmetic, 5 of 16
-//                     exponentials on the FMA pipe (cubic polynomial) instead of the special-function unit, writes p
-//                     back to TMEM as 16-bit pairs (the A operand of P V) and rescales the accumulator only when the
-//                     running max grew by more than 2^8 (exact: the final normalisation uses the same reference max).
-//   warp 12         : producer.  Issues the TMA loads of Q (double-buffered across items), K and V and stages, per key
-//                     tile, a "bias slab": a 128-byte-swizzled tile whose first two columns hold bias/scale split into
-//                     a high and a low 16-bit part (a large negative number past the segment end, which masks the
-//                     ragged tail).
-//   warps 13, 14, 15 : MMA issuer of query tile 0 / 1 / 2 (one elected lane issues).  S = Q K^T takes four K=16 steps
-//                     over the head dimension plus one K=16 step [1 1 0 ...] x [bias_hi bias_lo 0 ...]^T that adds
-//                     the per-key bias inside the tensor core; O += P V reads P from TMEM and V (N-major) from
-//                     shared memory.  S(j+1) is issued as soon as the softmax group holds S(j) in registers, P V as
-//                     soon as P(j) is staged.
-// TMEM columns: S_t [64 t, 64 t + 64), O_t [192 + 64 t, ...), P_t [384 + 32 t, ...), t = 0, 1, 2.
+//   warps 0-15     : softmax groups of query tiles 0 .. 3, four warps each.  Thread r owns score row r (TMEM lane r).  Per key
+//                     tile it pulls the 64 scores into registers, takes the row max with 3-input max, then
+//                     p = exp2(s * scale*log2e - m) in packed float32x2 arithmetic, a share of the exponentials on the FMA
+//                     pipe (cubic polynomial) instead of the special-function unit, writes p over the first half of its
+//                     scores as 16-bit pairs (the A operand of P V) and rescales the accumulator only when the running max
+//                     grew by more than 2^8 (exact: the final normalisation uses the same reference max).
+//   warp 16         : producer.  Issues the TMA loads of Q (double-buffered across items), K and V and stages, per key
+//                     tile, a "bias slab": a 64 x 16 tile whose first two columns hold bias/scale split into a high and a
+//                     low 16-bit part (a large negative number past the segment end, which masks the ragged tail).
+//   warps 17, 18    : MMA issuers of query tiles 0, 2 / 1, 3.  When P(j) of a tile is staged they issue O += P(j) V(j), with P
+//                     from TMEM and V (N-major) from shared memory, and right behind it S = Q K(j+1)^T over the same columns
+//                     (four K=16 steps over the head dimension plus one K=16 step [1 1 0 ...] x [bias_hi bias_lo 0 ...]^T that
+//                     adds the per-key bias inside the tensor core).  The tensor core runs them in order, so ONE barrier per
+//                     tile and direction carries a key step: "P staged" and "scores complete", which also says that the
+//                     accumulator is stable.
+// TMEM columns: S_t / P_t [64 t, 64 t + 64), O_t [256 + 64 t, ...), t = 0 .. 3.
+//
+// What bounds it: a key step of four tiles is ~2500 clocks (80,672 keys, 868 TFLOP/s): ~1470 of the tensor pipe (an M128 N64
+// K16 instruction with both operands in shared memory takes 48 clocks, with P in tensor memory 32), ~1400 of the
+// special-function unit and ~1600 issue slots per scheduler.  A tile alone takes ~1500 (softmax 850, hand-over and issue 260,
+// tensor work 370): the chain of a tile is serial, four tiles overlap.  The kernel before this one had three tiles with P beside
+// S (Q K(j+1)^T ran under the softmax of j), one issuer per tile and five barriers per tile and step: ~2080 clocks for three
+// tiles (786 TFLOP/s).  What made the difference are the issuers: with shared-memory and tensor-memory addresses known
+// at link time, one copy of the code per issuer and no vote or loop exit that depends on a wait, the nine instructions of a
+// tile and step are issued in ~190 clocks; with operands moved from ordinary registers they took ~590.
 //
 // Every wait on an mbarrier is bounded: after ~2^29 clock ticks the waiter raises the CTA's abort flag and the
 // library's device status word, every role falls through to the common exit, TMEM is released and the kernel
@@ -34,82 +43,57 @@ namespace come {
 
 namespace {
 
-constexpr int kTiles = 3;         // query tiles (128 rows each) per CTA and work item, one softmax warpgroup each
+constexpr int kTiles = 4;         // query tile slots (128 rows each) per CTA, one softmax warpgroup each
 constexpr int kBlockM = 128;
 constexpr int kBlockN = 64;       // keys per step
 constexpr int kHeadDim = 64;
-constexpr int kStages = 8;        // K/V ring slots, 8 KiB each
-constexpr int kSlabStages = 3;    // bias slab ring slots, 8 KiB each (only two 16-byte chunks per row are used)
+constexpr int kStages = 4;        // key tile ring: K, V (8 KiB each) and the bias slab of a key tile share a stage
 constexpr int kProducerWarp = 4 * kTiles;      // warps 0 .. 4*kTiles-1 are the softmax groups
-constexpr int kIssuerWarp0 = kProducerWarp + 1;  // one MMA issuer warp per query tile
-constexpr int kThreads = 32 * (kIssuerWarp0 + kTiles);  // 512: three softmax warpgroups + one producer / issuer warpgroup
+constexpr int kIssuers = 2;       // warps that issue the tensor-core work, two query tiles each
+constexpr int kIssuerWarp0 = kProducerWarp + 1;
+constexpr int kThreads = 32 * (kProducerWarp + 4);  // 640: four softmax warpgroups + one with the producer, the issuers and an idle warp
+static_assert(kTiles % kIssuers == 0 && 1 + kIssuers <= 4, "one warpgroup holds the producer and the issuers");
 // Launches with this many segments enumerate only the query blocks that exist (a prefix table in shared memory)
 constexpr int kMinPrefixSegs = 16, kMaxPrefixSegs = 2048;
 constexpr int kQTileBytes = kBlockM * kHeadDim * 2;   // 16384
 constexpr int kKvTileBytes = kBlockN * kHeadDim * 2;  // 8192
-// Tensor-memory columns: S_t (scores, float32) | O_t (accumulator, float32) | P_t (probabilities, 16-bit pairs)
-constexpr uint32_t kTmemS = 0, kTmemO = kTiles * kBlockN, kTmemP = kTmemO + kTiles * kHeadDim;
-static_assert(kTmemP + kTiles * (kBlockN / 2) <= 512, "tensor memory holds 512 columns");
+constexpr int kQSlabBytes = kBlockM * 16 * 2, kSlabBytes = kBlockN * 16 * 2;  // 16 columns of 16 bits
+// Tensor-memory columns: S_t (scores, float32), whose first half P_t (probabilities, 16-bit pairs) reuses | O_t (accumulator, float32)
+constexpr uint32_t kTmemS = 0, kTmemO = kTiles * kBlockN;
+static_assert(kTmemO + kTiles * kHeadDim <= 512, "tensor memory holds 512 columns");
 static_assert(kThreads % 128 == 0, "setmaxnreg works on whole warpgroups");
-static_assert(kMaxPrefixSegs % kThreads == 0, "every thread scans the same number of segments");
 constexpr uint32_t kTmemCols = 512;
 constexpr long long kWaitTicks = 1ll << 29;
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
 constexpr float kRescaleThreshold = 8.0f;  // log2 units
-// Which of the 16 score pairs of a 32-column quarter take the polynomial exp2 (bit i = pair i); the rest use the
-// special-function unit.  5 of 16 balanced the two pipes best in measurements of the two-tile predecessor; with three
-// tiles in flight shares from 0 to 6 of 16 measure within 2 % of each other.
+// Which of the 16 score pairs of a 32-column half take the polynomial exp2 (bit i = pair i); the rest use the
+// special-function unit.  0 / 3 / 4 / 5 of 16 on the polynomial route: 828 / 839 / 827 / 810 TFLOP/s at 24,576 keys, 624 / 666 /
+// 671 / 654 on 8 x 1374; the fewer take it, the less the kernel draws under the power cap.
 #ifndef COME_POLY_MASK
-#define COME_POLY_MASK 0x4924u
+#define COME_POLY_MASK 0x2108u
 #endif
 constexpr uint32_t kPolyPairs = COME_POLY_MASK;
 constexpr float kMasked = -3.0e38f;        // "minus infinity" of a masked key, still finite in bfloat16
 
-// Development builds (-DCOME_ATTN_TRACE) accumulate, per warp, the clocks spent in each kind of wait of the key loop and
-// leave them in a device array that come_debug_attn_trace() copies out; normal builds carry none of it.
-#ifdef COME_ATTN_TRACE
-constexpr int kTraceSlots = 12;
-__device__ unsigned long long g_attn_trace[256 * (kThreads / 32) * kTraceSlots];
-#define TRACE_DECL() long long tr_acc[kTraceSlots] = {}; long long tr_t = 0; (void)tr_t
-#define TRACE_BEGIN() tr_t = clock64()
-#define TRACE_END(slot) tr_acc[slot] += clock64() - tr_t
-#define TRACE_COUNT(slot, n) tr_acc[slot] += (n)
-#define TRACE_STAMP(slot, cond) do { if (cond) tr_acc[slot] = clock64(); } while (0)
-#define TRACE_FLUSH()                                                                                          \
-    do {                                                                                                       \
-        if ((threadIdx.x & 31) == 0 && blockIdx.x < 256)                                                       \
-            for (int i__ = 0; i__ < kTraceSlots; ++i__)                                                        \
-                g_attn_trace[(blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5)) * kTraceSlots + i__] = (unsigned long long)tr_acc[i__]; \
-    } while (0)
-#else
-#define TRACE_DECL()
-#define TRACE_BEGIN()
-#define TRACE_END(slot)
-#define TRACE_COUNT(slot, n)
-#define TRACE_STAMP(slot, cond)
-#define TRACE_FLUSH()
-#endif
-
 struct SharedStorage {
-    alignas(1024) uint8_t q[kTiles][2][kQTileBytes];        // [query tile][buffer]: the next item's Q is loaded ahead
-    alignas(1024) uint8_t kv[kStages][kKvTileBytes];
-    alignas(1024) uint8_t q_slab[kQTileBytes];              // columns 0,1 = 1.0, rest 0: the A side of the bias step
-    alignas(1024) uint8_t k_slab[kSlabStages][kKvTileBytes];  // columns 0,1 = bias/scale (hi, lo): the B side
-    alignas(8) uint64_t q_full[kTiles][2];                  // [query tile][buffer]
-    uint64_t q_empty[kTiles][2];
-    uint64_t q_slab_full;
+    alignas(1024) uint8_t q[2][kTiles][kQTileBytes];        // [buffer][query tile]: the next item's Q is loaded ahead
+    alignas(1024) uint8_t k[kStages][kKvTileBytes];
+    alignas(1024) uint8_t v[kStages][kKvTileBytes];
+    alignas(128) uint8_t q_slab[kQSlabBytes];               // columns 0,1 = 1.0, rest 0: the A side of the bias step
+    alignas(128) uint8_t k_slab[kStages][kSlabBytes];       // columns 0,1 = bias/scale (hi, lo), rest 0: the B side
+    alignas(8) uint64_t q_full[2];
+    uint64_t q_empty[2];
     uint64_t kv_full[kStages];
     uint64_t kv_empty[kStages];
-    uint64_t slab_full[kSlabStages];
-    uint64_t slab_empty[kSlabStages];
-    uint64_t s_full[kTiles];
+    uint64_t q_slab_full;
+    uint64_t s_full[kTiles];  // scores of a key tile complete (and, in order before them, P V of the key tile before)
     uint64_t p_full[kTiles];
-    uint64_t o_done[kTiles];
-    uint64_t s_empty[kTiles];
+    uint64_t o_done[kTiles];  // the last P V of an item complete
     uint32_t tmem_base;
     volatile uint32_t abort_flag;
     int scan_warp[kThreads / 32];
+    int height_sums[2 * kTiles];
 };
 // Launches that use the prefix table get (kMaxPrefixSegs + 1) ints of dynamic shared memory behind SharedStorage:
 // table[s] = query blocks of the segments before s (this launch's rows).
@@ -228,6 +212,16 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
         : "memory");
 }
 
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
+}
+
 __device__ __forceinline__ float max3(float a, float b, float c) {
     float d;
     asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
@@ -235,15 +229,19 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
 }
 // Makes generic-proxy shared-memory writes of this thread visible to the async proxy (tcgen05.mma operands).
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
-    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+// The bias slabs are K-major tiles without swizzle: 8-row x 16-byte core matrices, those of columns 0..7 first (8-row
+// groups 128 bytes apart), then those of columns 8..15.  Only columns 0 and 1 carry values; the rest stays zero.
+__device__ __forceinline__ uint32_t slab_offset(int r) { return (uint32_t)((r >> 3) * 128 + (r & 7) * 16); }
+__device__ __forceinline__ void st_shared_u32(uint32_t addr, uint32_t x) {
+    asm volatile("st.shared.b32 [%0], %1;" ::"r"(addr), "r"(x) : "memory");
 }
-// Row r of a slab (128-byte rows, 128-byte swizzle): logical 16-byte chunk c lives at physical chunk c ^ (r % 8).
-// Writes columns 0..7 = {v01 (two 16-bit values), 0 ...} and columns 8..15 = 0; the other chunks are never read.
-__device__ __forceinline__ void slab_write_row(uint32_t slab_addr, int r, uint32_t v01) {
-    const uint32_t row = slab_addr + (uint32_t)r * 128u;
-    st_shared_v4(row + (uint32_t)((0 ^ (r & 7)) << 4), v01, 0u, 0u, 0u);
-    st_shared_v4(row + (uint32_t)((1 ^ (r & 7)) << 4), 0u, 0u, 0u, 0u);
+__device__ __forceinline__ uint64_t make_slab_desc(uint32_t saddr, int rows) {
+    uint64_t d = 0;
+    d |= (uint64_t)((saddr & 0x3FFFF) >> 4);  // start address
+    d |= (uint64_t)(rows) << 16;              // leading byte offset: columns 0..7 to columns 8..15, rows * 16 bytes (in units of 16)
+    d |= (uint64_t)(128 >> 4) << 32;          // stride byte offset between 8-row groups
+    d |= (uint64_t)1 << 46;                   // descriptor version of sm_100; no swizzle
+    return d;
 }
 
 __device__ __forceinline__ float fast_exp2(float x) {
@@ -289,18 +287,17 @@ template <bool kBF16> __device__ __forceinline__ uint32_t pack2(float lo, float 
 }
 
 // Multiplies the 64 float32 accumulator columns of this thread's row by alpha (the rare rescale when a row's running
-// max grew past the threshold).  Out of line: inlined it would only bloat the hot loop.
-__device__ __noinline__ void scale_accumulator(uint32_t o_tmem, float alpha) {
-    uint32_t o[2][32];
-    tmem_ld32(o_tmem + 0, o[0]);
-    tmem_ld32(o_tmem + 32, o[1]);
-    tc_wait_ld();
+// max grew past the threshold), 16 columns at a time: the scores of the key tile stay in registers meanwhile.
+__device__ __forceinline__ void scale_accumulator(uint32_t o_tmem, float alpha) {
+#pragma unroll 1
+    for (int c = 0; c < kHeadDim; c += 16) {
+        uint32_t o[16];
+        tmem_ld16(o_tmem + c, o);
+        tc_wait_ld();
 #pragma unroll
-    for (int c = 0; c < 2; ++c)
-#pragma unroll
-        for (int i = 0; i < 32; ++i) o[c][i] = __float_as_uint(__uint_as_float(o[c][i]) * alpha);
-    tmem_st32(o_tmem + 0, o[0]);
-    tmem_st32(o_tmem + 32, o[1]);
+        for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+        tmem_st16(o_tmem + c, o);
+    }
 }
 
 // Shared-memory matrix descriptor of a tile whose rows are 128 bytes wide and 128-byte swizzled (what a TMA
@@ -324,12 +321,12 @@ __host__ __device__ constexpr uint32_t make_idesc(bool bf16, int M, int N, bool 
 }
 
 enum : uint32_t {
-    kErrQFull = 1u << 0, kErrKvFull = 1u << 1, kErrKvEmpty = 1u << 2, kErrSlabFull = 1u << 3, kErrSlabEmpty = 1u << 4,
-    kErrSFull = 1u << 5, kErrSEmpty = 1u << 6, kErrPFull = 1u << 7, kErrODone = 1u << 8,
+    kErrQFull = 1u << 0, kErrKvFull = 1u << 1, kErrKvEmpty = 1u << 2,
+    kErrSFull = 1u << 5, kErrPFull = 1u << 7, kErrODone = 1u << 8, kErrTmem = 1u << 9,
     kErrSelfTest = 1u << 15,  // raised by the wait self-test on purpose
 };
 
-// One work item = the (up to) kTiles 128-row query tiles [q_row0, q_row0 + kTiles * 128) of one (segment, head).
+// One work item = up to `tiles` 128-row query tiles [q_row0, q_row0 + tiles * 128) of one (segment, head).
 struct WorkItem {
     int head, s0, s1;   // head, key range of the segment
     int q_row0, q_hi;   // first query row of the item, end of the query rows this launch owns in the segment
@@ -339,11 +336,52 @@ struct WorkItem {
     int kpart;          // which share of the keys this item covers (launches that split the keys of their items), else 0
 };
 
-// Query blocks of segment `seg` that hold rows of this launch.
-__device__ __forceinline__ int segment_blocks(int seg, const int *__restrict__ cu, int q_begin, int q_end) {
+// 128-row query tiles of segment `seg` that hold rows of this launch.
+__device__ __forceinline__ int segment_tiles(int seg, const int *__restrict__ cu, int q_begin, int q_end) {
     const int rows = min(cu[seg + 1], q_end) - max(cu[seg], q_begin);
-    return rows > 0 ? (rows + kTiles * kBlockM - 1) / (kTiles * kBlockM) : 0;
+    return rows > 0 ? (rows + kBlockM - 1) / kBlockM : 0;
 }
+
+// Query tiles per work item.  A key step of an item costs less than in proportion to its tiles (the tiles share the SM's
+// units but each is a latency chain: 0.76 / 0.88 / 1.15 / 1.35 us with 1 / 2 / 3 / 4 tiles, 80,672 keys), so four tiles are
+// best where there are many items; but the items are dealt to the CTAs in rounds, and with few of them the height that
+// fills its last round wins: 6456 tokens x 16 heads take 215 us with 3 (272 items, 2 rounds) and 260 with 4 (208 items, also
+// 2 rounds); 3228 tokens 59 and 68 us; 2 segments of ~450 tokens 12.0 us with 1 and 16.8 with 4; 4 x 807 tokens 24 us with
+// 4 and 37 with 3.  The choice is the height with the least (rounds of items over the CTAs) x (mean cost of an item).  The
+// segments of a launch are known exactly on the device only, so every CTA makes the same choice from them (about 1 us of
+// the launch); the host makes it for one segment, and where every query tile gets a CTA of its own.
+__host__ __device__ __forceinline__ int step_cost(int n) { return n <= 0 ? 0 : n == 1 ? 64 : n == 2 ? 73 : n == 3 ? 96 : 113; }
+struct HeightSums {
+    int items[kTiles], cost[kTiles];  // [height - 1], of one head
+    __host__ __device__ __forceinline__ void add(int n) {
+#pragma unroll
+        for (int h = 1; h <= kTiles; ++h) {
+            items[h - 1] += (n + h - 1) / h;
+            cost[h - 1] += (n / h) * step_cost(h) + step_cost(n % h);
+        }
+    }
+    __device__ __forceinline__ void warp_sum() {
+#pragma unroll
+        for (int h = 0; h < kTiles; ++h) {
+            items[h] = __reduce_add_sync(0xffffffffu, items[h]);
+            cost[h] = __reduce_add_sync(0xffffffffu, cost[h]);
+        }
+    }
+    __host__ __device__ __forceinline__ int best(int num_heads, int ctas) const {
+        int height = kTiles;
+        float least = 3.0e38f;
+#pragma unroll
+        for (int h = kTiles; h >= 1; --h) {
+            const int rounds = (items[h - 1] * num_heads + ctas - 1) / ctas;
+            const float t = (float)rounds * (float)cost[h - 1] / (float)(items[h - 1] > 0 ? items[h - 1] : 1);
+            if (t < least) {
+                least = t;
+                height = h;
+            }
+        }
+        return height;
+    }
+};
 
 // Item -> (head, segment, query block).  With a prefix table (seg_prefix != nullptr) the items are exactly the query
 // blocks that exist, in (head, segment, block) order; without it every segment gets `nblk_x` slots and the surplus ones
@@ -352,7 +390,7 @@ __device__ __forceinline__ int segment_blocks(int seg, const int *__restrict__ c
 // inside the segment (attention of this GPU's rows to keys gathered from other GPUs); cu may then be NULL = [0, kv_total].
 template <bool kPrefix>
 __device__ __forceinline__ WorkItem decode_item(int item, int nblk_x, int nseg, const int *__restrict__ cu, int q_begin, int q_end,
-                                                const int *seg_prefix, int kv_total, bool q_free, int k_parts = 1) {
+                                                const int *seg_prefix, int kv_total, bool q_free, int tiles, int k_parts) {
     WorkItem w;
     int bx, seg;
     // Launches with k_parts > 1 (q_free only): consecutive items are the shares of the key tiles of one (head, block); every
@@ -387,9 +425,9 @@ __device__ __forceinline__ WorkItem decode_item(int item, int nblk_x, int nseg, 
     // slice when the query rows are sharded).  q / out / lse are indexed by (global row - q_begin); k / v by global row.
     const int q_lo = q_free ? q_begin : max(w.s0, q_begin);
     w.q_hi = q_free ? q_end : min(w.s1, q_end);
-    w.q_row0 = q_lo + bx * (kTiles * kBlockM);
+    w.q_row0 = q_lo + bx * (tiles * kBlockM);
     w.valid = w.q_row0 < w.q_hi;
-    w.n_mt = min(kTiles, (w.q_hi - w.q_row0 + kBlockM - 1) / kBlockM);  // query tiles with at least one valid row
+    w.n_mt = min(tiles, (w.q_hi - w.q_row0 + kBlockM - 1) / kBlockM);  // query tiles with at least one valid row
     w.n_kv = (seg_len + kBlockN - 1) / kBlockN;
     w.ragged_tail = (seg_len % kBlockN) != 0;
     if (k_parts > 1) {
@@ -418,20 +456,18 @@ __global__ void __launch_bounds__(kThreads, 1)
 attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                       const __grid_constant__ CUtensorMap map_v, const void *__restrict__ bias_ptr,
                       const int *__restrict__ cu, float scale_log2, float inv_scale, void *__restrict__ out_ptr, int64_t o_rs,
-                      float *__restrict__ lse, int q_begin, int q_end, int nblk_x, int nseg, int num_heads,
+                      float *__restrict__ lse, int q_begin, int q_end, int tiles, int max_rows, int nseg, int num_heads,
                       const int *__restrict__ max_len_dev, unsigned int *__restrict__ status, int kv_total, int q_free_flag,
                       int k_parts, long long part_o, long long part_l) {
     using T = typename std::conditional<kBF16, __nv_bfloat16, __half>::type;
-    extern __shared__ uint8_t smem_raw[];
-    SharedStorage &sh = *reinterpret_cast<SharedStorage *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    // the declared alignment makes the base, and with it every barrier address and matrix descriptor, a link-time constant
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    SharedStorage &sh = *reinterpret_cast<SharedStorage *>(smem_raw);
 
-    // The host sizes the work list from an upper bound of the longest segment.  A caller that cannot read the true
-    // length back (a captured graph serving every merge mask) passes a loose bound plus the true one in device memory:
-    // the work list then shrinks to the query blocks that can exist, and the round-robin over CTAs stays balanced.
-    if (max_len_dev != nullptr) {
-        const int m = min(max(*max_len_dev, 0), q_end - q_begin);
-        nblk_x = min(nblk_x, (m + kTiles * kBlockM - 1) / (kTiles * kBlockM));
-    }
+    // `max_rows` is the host's upper bound of the query rows of a segment.  A caller that cannot read the true length back
+    // (a captured graph serving every merge mask) passes a loose bound plus the true one in device memory.
+    if (max_len_dev != nullptr) max_rows = min(max_rows, max(*max_len_dev, 0));
+    int nblk_x = 0;  // slots per segment of a launch without the prefix table
     // Work list.  Launches with many segments (kMinPrefixSegs .. kMaxPrefixSegs): every CTA scans the segments' query-block
     // counts into shared memory and the items are exactly the blocks that exist.  With ragged segments a list with one
     // slot per (segment, maximal block index) unbalances the round-robin: the empty slots all carry the same block index,
@@ -440,12 +476,37 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     constexpr bool use_prefix = kPrefix;  // the host instantiates and sizes the shared memory by the segment count
     int *prefix_table = reinterpret_cast<int *>(reinterpret_cast<uint8_t *>(&sh) + sizeof(SharedStorage));
     if constexpr (kPrefix) {
-        constexpr int kPer = kMaxPrefixSegs / kThreads;  // consecutive segments per thread
+        constexpr int kPer = (kMaxPrefixSegs + kThreads) / kThreads;  // consecutive segments per thread
         int local[kPer], sum = 0;
+        HeightSums hs = {};
 #pragma unroll
         for (int i = 0; i < kPer; ++i) {
             const int sg = threadIdx.x * kPer + i;
-            local[i] = sg < nseg ? segment_blocks(sg, cu, q_begin, q_end) : 0;
+            local[i] = sg < nseg ? segment_tiles(sg, cu, q_begin, q_end) : 0;
+            hs.add(local[i]);
+        }
+        if (tiles == 0) {
+            if (threadIdx.x < 2 * kTiles) sh.height_sums[threadIdx.x] = 0;
+            __syncthreads();
+            hs.warp_sum();
+            if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+                for (int h = 0; h < kTiles; ++h) {
+                    atomicAdd(&sh.height_sums[h], hs.items[h]);
+                    atomicAdd(&sh.height_sums[kTiles + h], hs.cost[h]);
+                }
+            }
+            __syncthreads();
+#pragma unroll
+            for (int h = 0; h < kTiles; ++h) {
+                hs.items[h] = sh.height_sums[h];
+                hs.cost[h] = sh.height_sums[kTiles + h];
+            }
+            tiles = hs.best(num_heads, gridDim.x);
+        }
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) {
+            local[i] = (local[i] + tiles - 1) / tiles;
             sum += local[i];
         }
         int incl = sum;
@@ -464,8 +525,21 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
             if (sg <= nseg) prefix_table[sg] = before;
             before += local[i];
         }
-        if (nseg == kMaxPrefixSegs && threadIdx.x == kThreads - 1) prefix_table[kMaxPrefixSegs] = before;  // the grand total
         __syncthreads();
+    }
+    if constexpr (!kPrefix) {
+        const int lane_seg = threadIdx.x & 31;
+        if (tiles == 0) {  // fewer than kMinPrefixSegs segments: a lane each, every warp on its own
+            int n = lane_seg < nseg ? segment_tiles(lane_seg, cu, q_begin, q_end) : 0;
+            n = min(n, (max_rows + kBlockM - 1) / kBlockM);
+            HeightSums hs = {};
+            hs.add(n);
+            hs.warp_sum();
+            tiles = hs.best(num_heads, gridDim.x);
+            nblk_x = (__reduce_max_sync(0xffffffffu, n) + tiles - 1) / tiles;
+        } else {
+            nblk_x = (max_rows + tiles * kBlockM - 1) / (tiles * kBlockM);
+        }
     }
     const int *seg_prefix = use_prefix ? prefix_table : nullptr;
     const int total_items = (use_prefix ? prefix_table[nseg] * num_heads : nblk_x * nseg * num_heads) * k_parts;
@@ -479,23 +553,18 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     if (threadIdx.x == 0) {
         // an earlier CTA that gave up leaves the status word raised: later CTAs then skip their work
         sh.abort_flag = (*(volatile unsigned int *)status != 0) ? 1u : 0u;
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&sh.q_full[i], 1);
+            mbar_init(&sh.q_empty[i], kIssuers);
+        }
         for (int i = 0; i < kTiles; ++i) {
-            for (int b = 0; b < 2; ++b) {
-                mbar_init(&sh.q_full[i][b], 1);
-                mbar_init(&sh.q_empty[i][b], 1);
-            }
             mbar_init(&sh.s_full[i], 1);
             mbar_init(&sh.p_full[i], kBlockM);
             mbar_init(&sh.o_done[i], 1);
-            mbar_init(&sh.s_empty[i], kBlockM);
         }
         for (int i = 0; i < kStages; ++i) {
-            mbar_init(&sh.kv_full[i], 1);
-            mbar_init(&sh.kv_empty[i], kTiles);  // released by every issuer warp (an idle one arrives without an MMA)
-        }
-        for (int i = 0; i < kSlabStages; ++i) {
-            mbar_init(&sh.slab_full[i], 1);
-            mbar_init(&sh.slab_empty[i], kTiles);
+            mbar_init(&sh.kv_full[i], 2);   // the TMA loads and the bias slab
+            mbar_init(&sh.kv_empty[i], kIssuers);
         }
         mbar_init(&sh.q_slab_full, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -507,282 +576,268 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = sh.tmem_base;
-    // Register budget: the producer / issuer warpgroup needs few registers and hands its share to the three softmax
-    // warpgroups (12 x 32 x 152 + 4 x 32 x 56 = 65536).  Each role branch below starts with its setmaxnreg; every warp
-    // of a warpgroup has to execute it.
-    const bool dead = sh.abort_flag != 0;  // read after the barrier: uniform for the CTA
+    // All of the SM's tensor memory is allocated, so its base is column 0: the tensor-memory addresses are constants.
+    constexpr uint32_t tmem = 0;
+    // Register budget: the producer / issuer warpgroup needs few registers and hands its share to the softmax warpgroups
+    // (640 x 96 at launch = 61440 = 16 x 32 x 104 + 4 x 32 x 64).  Every warp of a warpgroup executes its setmaxnreg.
+    const bool dead = sh.abort_flag != 0 || sh.tmem_base != tmem;  // read after the barrier: uniform for the CTA
 
     if (dead) {
-        // fall through to the common exit
-    } else if (warp == kProducerWarp) {
-        // ===== producer =====================================================================================
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
-        const T *bias = reinterpret_cast<const T *>(bias_ptr);
-        bool ok = true;
-        {   // the constant A side of the bias step: columns 0 and 1 are 1.0.  Both slabs are bfloat16 whatever the
-            // q/k/v dtype (the bias step is an MMA instruction of its own): bias/scale and the mask value need its range.
-            const uint32_t ones = pack2<true>(1.0f, 1.0f);
-            const uint32_t qs = smem_u32(sh.q_slab);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) slab_write_row(qs, lane * 4 + i, ones);
-            fence_proxy_async();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&sh.q_slab_full);
-        }
-        int it = 0;            // K/V ring position, advanced once per K or V tile in the order K0 V0 K1 V1 ...
-        int slab_it = 0;       // bias slab ring position, advanced once per key tile that uses the bias step
-        int q_uses[kTiles] = {};  // items that loaded query tile t so far (buffer and phase of q_full / q_empty)
-        for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x) {
-            const WorkItem w = decode_item<kPrefix>(item, nblk_x, nseg, cu, q_begin, q_end, seg_prefix, kv_total, q_free, k_parts);
-            if (!w.valid) continue;
-            if (lane == 0) {
-                for (int t = 0; t < w.n_mt && ok; ++t) {
-                    // Use n of query tile t goes to buffer n & 1, which is free once the last Q K^T of use n - 2 has completed:
-                    // the query tiles of the next item are in flight while the current item is still being computed.
-                    const int n = q_uses[t], b = n & 1;
-                    if (n >= 2) ok = mbar_wait(&sh.q_empty[t][b], ((n >> 1) - 1) & 1, sh, status, kErrQFull);
+        if (threadIdx.x == 0 && sh.tmem_base != tmem) atomicOr(status, kErrTmem);
+    } else if (warp >= kProducerWarp) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+        if (warp == kProducerWarp) {
+            // ===== producer =================================================================================
+            const T *bias = reinterpret_cast<const T *>(bias_ptr);
+            bool ok = true;
+            {   // the constant A side of the bias step: columns 0 and 1 are 1.0.  Both slabs are bfloat16 whatever the
+                // q/k/v dtype (the bias step is an MMA instruction of its own): bias/scale and the mask value need its range.
+                const uint32_t ones = pack2<true>(1.0f, 1.0f);
+                const uint32_t qs = smem_u32(sh.q_slab), ks = smem_u32(sh.k_slab);
+                for (int i = lane * 4; i < kQSlabBytes; i += 128) st_shared_u32(qs + i, 0u);
+                for (int i = lane * 4; i < kStages * kSlabBytes; i += 128) st_shared_u32(ks + i, 0u);
+                __syncwarp();
+                for (int i = lane; i < kBlockM; i += 32) st_shared_u32(qs + slab_offset(i), ones);
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&sh.q_slab_full);
+            }
+            int it = 0;      // ring position, advanced once per key tile
+            int q_uses = 0;  // items loaded so far (buffer and phase of q_full / q_empty)
+            for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x) {
+                const WorkItem w = decode_item<kPrefix>(item, nblk_x, nseg, cu, q_begin, q_end, seg_prefix, kv_total, q_free, tiles, k_parts);
+                if (!w.valid) continue;
+                if (lane == 0) {
+                    // Item n uses Q buffer n & 1, free once the last tensor-core work of item n - 2 has completed: the next
+                    // item's query tiles are in flight while the current item is being computed.
+                    const int b = q_uses & 1;
+                    if (q_uses >= 2) ok = mbar_wait(&sh.q_empty[b], ((q_uses >> 1) - 1) & 1, sh, status, kErrQFull);
                     if (ok) {
-                        mbar_arrive_expect_tx(&sh.q_full[t][b], kQTileBytes);
-                        tma_load_3d(sh.q[t][b], &map_q, 0, w.head, w.q_row0 - q_begin + t * kBlockM, &sh.q_full[t][b]);
+                        mbar_arrive_expect_tx(&sh.q_full[b], w.n_mt * kQTileBytes);
+                        for (int t = 0; t < w.n_mt; ++t)
+                            tma_load_3d(sh.q[b][t], &map_q, 0, w.head, w.q_row0 - q_begin + t * kBlockM, &sh.q_full[b]);
                     }
                 }
-            }
-            for (int t = 0; t < w.n_mt; ++t) ++q_uses[t];
-            ok = __all_sync(0xffffffffu, ok);
-            for (int j = 0; j < w.n_kv && ok; ++j) {
-                if (uses_slab(w, j)) {
-                    const int bs = slab_it % kSlabStages;
-                    ok = mbar_wait(&sh.slab_empty[bs], ((slab_it / kSlabStages) & 1) ^ 1, sh, status, kErrSlabEmpty);
-                    ok = __all_sync(0xffffffffu, ok);
-                    if (!ok) break;
-                    const uint32_t ks = smem_u32(sh.k_slab[bs]);
+                ++q_uses;
+                ok = __all_sync(0xffffffffu, ok);
+                // bias of the lane's keys, fetched one key tile ahead of its use
+                float next_bias[kBlockN / 32];
+                auto fetch_bias = [&](int j) {
 #pragma unroll
                     for (int i = 0; i < kBlockN / 32; ++i) {
-                        const int r = lane * (kBlockN / 32) + i;
-                        const int key = w.s0 + j * kBlockN + r;
-                        float hi = kMasked, lo = 0.0f;
-                        if (key < w.s1) {
-                            const float b = has_bias ? Elem<T>::to_f32(bias[key]) * inv_scale : 0.0f;
-                            hi = __bfloat162float(__float2bfloat16_rn(b));
-                            lo = b - hi;
-                        }
-                        slab_write_row(ks, r, pack2<true>(hi, lo));
+                        const int key = w.s0 + j * kBlockN + i * 32 + lane;
+                        next_bias[i] = key < w.s1 && has_bias ? Elem<T>::to_f32(bias[key]) : 0.0f;
                     }
-                    fence_proxy_async();
+                };
+                fetch_bias(0);
+                for (int j = 0; j < w.n_kv && ok; ++j, ++it) {
+                    const int st = it % kStages;
+                    ok = mbar_wait(&sh.kv_empty[st], ((it / kStages) & 1) ^ 1, sh, status, kErrKvEmpty);
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) break;
+                    if (lane == 0) {
+                        mbar_arrive_expect_tx(&sh.kv_full[st], 2 * kKvTileBytes);
+                        tma_load_3d(sh.k[st], &map_k, 0, w.head, w.s0 + j * kBlockN, &sh.kv_full[st]);
+                        tma_load_3d(sh.v[st], &map_v, 0, w.head, w.s0 + j * kBlockN, &sh.kv_full[st]);
+                    }
+                    if (uses_slab(w, j)) {
+                        const uint32_t ks = smem_u32(sh.k_slab[st]);
+#pragma unroll
+                        for (int i = 0; i < kBlockN / 32; ++i) {
+                            const bool masked = w.s0 + j * kBlockN + i * 32 + lane >= w.s1;
+                            const float b = next_bias[i] * inv_scale;
+                            const float hi = masked ? kMasked : __bfloat162float(__float2bfloat16_rn(b));
+                            st_shared_u32(ks + slab_offset(i * 32 + lane), pack2<true>(hi, masked ? 0.0f : b - hi));
+                        }
+                        fence_proxy_async();
+                    }
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(&sh.slab_full[bs]);
-                    ++slab_it;
+                    if (lane == 0) mbar_arrive(&sh.kv_full[st]);
+                    if (j + 1 < w.n_kv) fetch_bias(j + 1);
                 }
-                if (lane == 0) {
-#pragma unroll
-                    for (int kv = 0; kv < 2 && ok; ++kv) {  // K tile, then V tile of the same keys
-                        const int stage = (it + kv) % kStages;
-                        ok = mbar_wait(&sh.kv_empty[stage], (((it + kv) / kStages) & 1) ^ 1, sh, status, kErrKvEmpty);
-                        if (ok) {
-                            mbar_arrive_expect_tx(&sh.kv_full[stage], kKvTileBytes);
-                            tma_load_3d(sh.kv[stage], kv == 0 ? &map_k : &map_v, 0, w.head, w.s0 + j * kBlockN, &sh.kv_full[stage]);
-                        }
-                    }
-                }
-                ok = __all_sync(0xffffffffu, ok);
-                it += 2;
             }
-        }
-    } else if (warp >= kIssuerWarp0) {
-        // ===== MMA issuer of query tile t (all lanes run the loop, one elected lane issues) ================
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
-        const int t = warp - kIssuerWarp0;
-        constexpr uint32_t idesc_qk = make_idesc(kBF16, kBlockM, kBlockN, false);
-        constexpr uint32_t idesc_slab = make_idesc(true, kBlockM, kBlockN, false);
-        constexpr uint32_t idesc_pv = make_idesc(kBF16, kBlockM, kHeadDim, true);
-        const uint64_t q_desc0 = make_smem_desc(smem_u32(sh.q[t][0]));  // buffer b: + b * (kQTileBytes >> 4)
-        const uint64_t q_slab_desc = make_smem_desc(smem_u32(sh.q_slab));
-        const uint64_t kv_desc0 = make_smem_desc(smem_u32(sh.kv[0]));       // slot i: + i * (kKvTileBytes >> 4)
-        const uint64_t k_slab_desc0 = make_smem_desc(smem_u32(sh.k_slab[0]));
-        const uint32_t s_tmem = tmem + kTmemS + t * kBlockN;
-        const uint32_t o_tmem = tmem + kTmemO + t * kHeadDim;
-        const uint32_t p_tmem = tmem + kTmemP + t * (kBlockN / 2);
-        bool ok = mbar_wait(&sh.q_slab_full, 0, sh, status, kErrQFull);
-        ok = __all_sync(0xffffffffu, ok);
-        int it = 0;        // K/V ring position at the start of the current item (same count as the producer's)
-        int slab_it = 0;   // bias slab ring position
-        int step = 0;      // key tiles this query tile has processed so far (phase of s_full / s_empty / p_full / o_done)
-        int q_uses = 0;    // items in which this query tile was active (phase of q_full / q_empty)
-        TRACE_DECL();
-#ifdef COME_ATTN_TRACE
-        const long long tr_start = clock64();
-#endif
-        for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x) {
-            const WorkItem w = decode_item<kPrefix>(item, nblk_x, nseg, cu, q_begin, q_end, seg_prefix, kv_total, q_free, k_parts);
-            if (!w.valid) continue;
-            if (t >= w.n_mt) {
-                // This query tile is empty in this item: release the K/V and slab slots without using them, so that the
-                // rings' arrival counts do not depend on the item.
-                for (int j = 0; j < w.n_kv && ok; ++j) {
-#pragma unroll
-                    for (int kv = 0; kv < 2 && ok; ++kv) {
-                        const int x = it + 2 * j + kv, slot = x % kStages;
-                        ok = mbar_wait(&sh.kv_full[slot], (x / kStages) & 1, sh, status, kErrKvFull);
-                        ok = __all_sync(0xffffffffu, ok);
-                        if (ok && lane == 0) mbar_arrive(&sh.kv_empty[slot]);
-                    }
-                    if (ok && uses_slab(w, j)) {
-                        const int bs = slab_it % kSlabStages;
-                        ok = mbar_wait(&sh.slab_full[bs], (slab_it / kSlabStages) & 1, sh, status, kErrSlabFull);
-                        ok = __all_sync(0xffffffffu, ok);
-                        if (ok && lane == 0) mbar_arrive(&sh.slab_empty[bs]);
-                        ++slab_it;
-                    }
-                }
-                it += 2 * w.n_kv;
-                continue;
-            }
-            const int qb = q_uses & 1;
-            ok = mbar_wait(&sh.q_full[t][qb], (q_uses >> 1) & 1, sh, status, kErrQFull);
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok) break;
-            const uint64_t q_desc = q_desc0 + (uint64_t)(qb * (kQTileBytes >> 4));
-            // S(0), then per key tile j: S(j+1) = Q K_(j+1)^T as soon as the softmax group has read S(j) into registers,
-            // and O += P(j) V_j as soon as P(j) is staged.  Ring slot of K_j is 2j, of V_j is 2j+1 (from `it`).  The other
-            // query tile's issuer runs the same loop independently.
-            // S(jj) = Q K_jj^T (+ the bias step): what it waits for, and its instructions
-            auto wait_s = [&](int jj) -> bool {
-                const int k_it = it + 2 * jj, k_slot = k_it % kStages;
-                const int bs = slab_it % kSlabStages;
-                TRACE_BEGIN();
-                bool good = mbar_wait(&sh.kv_full[k_slot], (k_it / kStages) & 1, sh, status, kErrKvFull);
-                if (good && uses_slab(w, jj)) good = mbar_wait(&sh.slab_full[bs], (slab_it / kSlabStages) & 1, sh, status, kErrSlabFull);
-                TRACE_END(0);
-                TRACE_BEGIN();
-                // the softmax group must have pulled the previous scores (also those of the previous item) out of S
-                if (good && step + jj > 0) good = mbar_wait(&sh.s_empty[t], (step + jj - 1) & 1, sh, status, kErrSEmpty);
-                TRACE_END(1);
-                TRACE_STAMP(8, step + jj == 65);
-                return __all_sync(0xffffffffu, good);
-            };
-            auto emit_s = [&](int jj) {
-                const int k_it = it + 2 * jj, k_slot = k_it % kStages;
-                const bool slab = uses_slab(w, jj);
-                const int bs = slab_it % kSlabStages;
-                const uint64_t k_desc = kv_desc0 + (uint64_t)(k_slot * (kKvTileBytes >> 4));
-                if (elect_one()) {  // one lane issues the whole group: a single election and branch instead of one per instruction
-                    tc_mma_ss_1(s_tmem, q_desc + 0, k_desc + 0, idesc_qk, 0u);
-                    tc_mma_ss_1(s_tmem, q_desc + 2, k_desc + 2, idesc_qk, 1u);
-                    tc_mma_ss_1(s_tmem, q_desc + 4, k_desc + 4, idesc_qk, 1u);
-                    tc_mma_ss_1(s_tmem, q_desc + 6, k_desc + 6, idesc_qk, 1u);
-                    if (slab) tc_mma_ss_1(s_tmem, q_slab_desc, k_slab_desc0 + (uint64_t)(bs * (kKvTileBytes >> 4)), idesc_slab, 1u);
+        } else if (warp < kIssuerWarp0 + kIssuers) {
+            // ===== MMA issuers: query tiles first, first + kIssuers, ... ====================================
+            // One copy of the code per issuer and uniform control flow, so that the operands of the tensor-core instructions
+            // are constants or uniform registers; one elected lane issues a tile's group.
+            auto run = [&](auto first_c) {
+                constexpr int first = decltype(first_c)::value;
+                constexpr uint32_t idesc_qk = make_idesc(kBF16, kBlockM, kBlockN, false);
+                constexpr uint32_t idesc_slab = make_idesc(true, kBlockM, kBlockN, false);
+                constexpr uint32_t idesc_pv = make_idesc(kBF16, kBlockM, kHeadDim, true);
+                const uint64_t q_desc0 = make_smem_desc(smem_u32(sh.q));
+                const uint64_t q_slab_desc = make_slab_desc(smem_u32(sh.q_slab), kBlockM);
+                const uint64_t k_desc0 = make_smem_desc(smem_u32(sh.k));
+                const uint64_t v_desc0 = make_smem_desc(smem_u32(sh.v));
+                const uint64_t k_slab_desc0 = make_slab_desc(smem_u32(sh.k_slab), kBlockN);
+                // S_t = Q_t K^T (+ the bias step) from ring stage st and Q buffer b
+                auto qk = [&](int t, uint32_t st, uint32_t b, bool slab) {
+                    const uint32_t s_tmem = tmem + kTmemS + t * kBlockN;
+                    const uint64_t qd = q_desc0 + (uint64_t)((b * kTiles + t) * (kQTileBytes >> 4));
+                    const uint64_t kd = k_desc0 + (uint64_t)(st * (kKvTileBytes >> 4));
+                    tc_mma_ss_1(s_tmem, qd + 0, kd + 0, idesc_qk, 0u);
+                    tc_mma_ss_1(s_tmem, qd + 2, kd + 2, idesc_qk, 1u);
+                    tc_mma_ss_1(s_tmem, qd + 4, kd + 4, idesc_qk, 1u);
+                    tc_mma_ss_1(s_tmem, qd + 6, kd + 6, idesc_qk, 1u);
+                    if (slab) tc_mma_ss_1(s_tmem, q_slab_desc, k_slab_desc0 + (uint64_t)(st * (kSlabBytes >> 4)), idesc_slab, 1u);
                     tc_commit_1(&sh.s_full[t]);
-                    tc_commit_1(&sh.kv_empty[k_slot]);
-                    if (slab) tc_commit_1(&sh.slab_empty[bs]);
-                    if (jj == w.n_kv - 1) tc_commit_1(&sh.q_empty[t][qb]);
-                }
-                __syncwarp();
-                if (slab) ++slab_it;
-                TRACE_STAMP(11, step + jj == 65);
-            };
-            // O += P(j) V_j: what it waits for, and its instructions
-            auto wait_pv = [&](int j) -> bool {
-                const int v_it = it + 2 * j + 1, v_slot = v_it % kStages;
-                TRACE_BEGIN();
-                bool good = mbar_wait(&sh.kv_full[v_slot], (v_it / kStages) & 1, sh, status, kErrKvFull);
-                TRACE_END(2);
-                TRACE_BEGIN();
-                if (good) good = mbar_wait(&sh.p_full[t], (step + j) & 1, sh, status, kErrPFull);
-                TRACE_END(3);
-                TRACE_COUNT(5, 1);
-                TRACE_STAMP(9, step + j == 64);
-                return __all_sync(0xffffffffu, good);
-            };
-            auto emit_pv = [&](int j) {
-                const int v_it = it + 2 * j + 1, v_slot = v_it % kStages;
-                const uint64_t v_desc = kv_desc0 + (uint64_t)(v_slot * (kKvTileBytes >> 4));
-                // 16 keys per instruction: 8 columns of 16-bit pairs of P, 16 rows (2048 bytes) of the V tile
-                if (elect_one()) {
+                };
+                // O_t += P_t V: 16 keys per instruction = 8 columns of 16-bit pairs of P, 16 rows (2048 bytes) of the V tile
+                auto pv = [&](int t, uint32_t st, uint32_t accumulate) {
+                    const uint32_t o_tmem = tmem + kTmemO + t * kHeadDim, p_tmem = tmem + kTmemS + t * kBlockN;
+                    const uint64_t vd = v_desc0 + (uint64_t)(st * (kKvTileBytes >> 4));
 #pragma unroll
                     for (int i = 0; i < kBlockN / 16; ++i)
-                        tc_mma_ts_1(o_tmem, p_tmem + 8 * i, v_desc + (uint64_t)(i * 128), idesc_pv, (j > 0 || i > 0) ? 1u : 0u);
-                    tc_commit_1(&sh.o_done[t]);
-                    tc_commit_1(&sh.kv_empty[v_slot]);
-                }
-                __syncwarp();
-                TRACE_STAMP(10, step + j == 64);
-            };
-            ok = wait_s(0);
-            if (ok) {
-                tc_fence_after();
-                emit_s(0);
-            }
-            for (int j = 0; j < w.n_kv && ok; ++j) {
-                if (j + 1 < w.n_kv) {
-                    ok = wait_s(j + 1);
-                    if (!ok) break;
+                        tc_mma_ts_1(o_tmem, p_tmem + 8 * i, vd + (uint64_t)(i * 128), idesc_pv, i > 0 ? 1u : accumulate);
+                };
+                struct Item {
+                    int n_mt, n_kv;
+                    bool ragged;
+                };
+                auto next_valid = [&](int &item, Item &x) -> bool {
+                    for (; item < total_items; item += gridDim.x) {
+                        const WorkItem w = decode_item<kPrefix>(item, nblk_x, nseg, cu, q_begin, q_end, seg_prefix, kv_total, q_free, tiles, k_parts);
+                        if (w.valid) {
+                            x = Item{w.n_mt, w.n_kv, w.ragged_tail};
+                            return true;
+                        }
+                    }
+                    return false;
+                };
+                auto item_slab = [&](const Item &x, int j) { return has_bias || (x.ragged && j == x.n_kv - 1); };
+                uint32_t st = 0, kv_phase = 0;  // ring stage of the current key tile; phase of kv_full for the stage after it
+                uint32_t p_phase = 0;           // bit t: phase of p_full[t]
+                uint32_t qb = 0, q_phase = 0;   // Q buffer of the current item; bit b: phase of q_full[b]
+                int items = 0;                  // items done
+                int item = blockIdx.x;
+                Item w, nx;
+                bool have = next_valid(item, w);
+                mbar_wait(&sh.q_slab_full, 0, sh, status, kErrQFull);
+                if (have) {  // the first scores of the first item; later items' first scores are issued with the last P V before them
+                    mbar_wait(&sh.q_full[0], 0, sh, status, kErrQFull);
+                    mbar_wait(&sh.kv_full[0], 0, sh, status, kErrKvFull);
+                    q_phase ^= 1u;
+                    __syncwarp();
                     tc_fence_after();
-                    emit_s(j + 1);
+                    if (elect_one()) {
+#pragma unroll
+                        for (int t = first; t < kTiles; t += kIssuers)
+                            if (t < w.n_mt) qk(t, 0, 0, item_slab(w, 0));
+                    }
+                    __syncwarp();
                 }
-                ok = wait_pv(j);
-                if (!ok) break;
-                tc_fence_after();
-                emit_pv(j);
-            }
-            it += 2 * w.n_kv;
-            step += w.n_kv;
-            ++q_uses;
+                // A wait that gives up does not end the key loop (its result would make the loop's control flow, and with it
+                // the operands, non-uniform): the remaining waits of the item return at once and the item loop ends.
+                while (have) {
+                    // key tiles with a successor in the same item
+                    for (int j = 0; j < w.n_kv - 1; ++j) {
+                        const uint32_t st2 = (st + 1) % kStages;
+                        if (st2 == 0) kv_phase ^= 1u;
+                        mbar_wait(&sh.kv_full[st2], kv_phase, sh, status, kErrKvFull);
+                        const bool slab2 = item_slab(w, j + 1);
+#pragma unroll
+                        for (int t = first; t < kTiles; t += kIssuers) {
+                            if (t < w.n_mt) {
+                                // O_t += P_t V, then the next scores of the tile over P_t: the tensor core executes them in order
+                                mbar_wait(&sh.p_full[t], (p_phase >> t) & 1, sh, status, kErrPFull);
+                                p_phase ^= 1u << t;
+                                __syncwarp();
+                                tc_fence_after();
+                                if (elect_one()) {
+                                    pv(t, st, j > 0 ? 1u : 0u);
+                                    qk(t, st2, qb, slab2);
+                                }
+                                __syncwarp();
+                            }
+                        }
+                        if (elect_one()) tc_commit_1(&sh.kv_empty[st]);
+                        __syncwarp();
+                        st = st2;
+                    }
+                    // last key tile: its scores' successor is the first key tile of the next item, if there is one
+                    int item2 = item + gridDim.x;
+                    const bool have2 = next_valid(item2, nx);
+                    const uint32_t st2 = (st + 1) % kStages;
+                    bool slab2 = false;
+                    if (st2 == 0) kv_phase ^= 1u;
+                    if (have2) {
+                        mbar_wait(&sh.kv_full[st2], kv_phase, sh, status, kErrKvFull);
+                        mbar_wait(&sh.q_full[qb ^ 1], (q_phase >> (qb ^ 1)) & 1, sh, status, kErrQFull);
+                        q_phase ^= 1u << (qb ^ 1);
+                        slab2 = item_slab(nx, 0);
+                    } else {
+                        nx.n_mt = 0;
+                    }
+                    const uint32_t multi = w.n_kv > 1 ? 1u : 0u;
+#pragma unroll
+                    for (int t = first; t < kTiles; t += kIssuers) {
+                        if (t < w.n_mt) {
+                            mbar_wait(&sh.p_full[t], (p_phase >> t) & 1, sh, status, kErrPFull);
+                            p_phase ^= 1u << t;
+                        }
+                        __syncwarp();
+                        tc_fence_after();
+                        if (elect_one()) {
+                            if (t < w.n_mt) {
+                                pv(t, st, multi);
+                                tc_commit_1(&sh.o_done[t]);
+                            }
+                            if (t < nx.n_mt) qk(t, st2, qb ^ 1, slab2);
+                        }
+                        __syncwarp();
+                    }
+                    if (elect_one()) {
+                        tc_commit_1(&sh.kv_empty[st]);
+                        tc_commit_1(&sh.q_empty[qb]);
+                    }
+                    __syncwarp();
+                    st = st2;
+                    qb ^= 1u;
+                    ++items;
+                    item = item2;
+                    w = nx;
+                    have = have2 && __all_sync(0xffffffffu, sh.abort_flag == 0);
+                }
+                // the last commits have arrived before the CTA may end
+                if (items > 0) mbar_wait(&sh.q_empty[qb ^ 1], ((items - 1) >> 1) & 1, sh, status, kErrQFull);
+                __syncwarp();
+            };
+            if (warp == kIssuerWarp0) run(std::integral_constant<int, 0>{});
+            else run(std::integral_constant<int, 1>{});
         }
-#ifdef COME_ATTN_TRACE
-        tr_acc[4] = clock64() - tr_start;
-#endif
-        TRACE_FLUSH();
-        __syncwarp();
     } else {
         // ===== softmax group of query tile t ================================================================
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 152;");
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
         const int t = warp >> 2;
         const int r = threadIdx.x & 127;                          // row inside the tile == TMEM lane
         const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
-        const uint32_t s_tmem = tmem + lane_addr + kTmemS + t * kBlockN;
+        const uint32_t s_tmem = tmem + lane_addr + kTmemS + t * kBlockN;  // P goes over the first half of the scores
         const uint32_t o_tmem = tmem + lane_addr + kTmemO + t * kHeadDim;
-        const uint32_t p_tmem = tmem + lane_addr + kTmemP + t * (kBlockN / 2);
         bool ok = true;
-        int step = 0;  // key tiles processed so far by this query tile: phase of s_full / s_empty / p_full / o_done
-        TRACE_DECL();
-#ifdef COME_ATTN_TRACE
-        const long long tr_start = clock64();
-#endif
+        uint32_t s_phase = 0, o_phase = 0;
         for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x) {
-            const WorkItem w = decode_item<kPrefix>(item, nblk_x, nseg, cu, q_begin, q_end, seg_prefix, kv_total, q_free, k_parts);
+            const WorkItem w = decode_item<kPrefix>(item, nblk_x, nseg, cu, q_begin, q_end, seg_prefix, kv_total, q_free, tiles, k_parts);
             if (!w.valid || t >= w.n_mt) continue;
             const int n_kv = w.n_kv;
-            const int row = w.q_row0 + t * kBlockM + r;
             float m_ref = -INFINITY, l = 0.0f;  // reference max (log2 units, scale applied) and running sum
 
-            for (int j = 0; j < n_kv && ok; ++j) {
-                TRACE_BEGIN();
-                ok = mbar_wait(&sh.s_full[t], (step + j) & 1, sh, status, kErrSFull);
-                TRACE_END(0);
-                TRACE_COUNT(5, 1);
-                TRACE_STAMP(8, step + j == 64);
-                TRACE_STAMP(9, step + j == 65);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
+            for (int j = 0; j < n_kv; ++j) {
+                // The scores of key tile j are complete, and with them (in order) P V of key tile j - 1: the accumulator is
+                // stable and P may be overwritten.
+                ok = mbar_wait(&sh.s_full[t], s_phase, sh, status, kErrSFull);
+                s_phase ^= 1u;
+                __syncwarp();
                 tc_fence_after();
-                TRACE_BEGIN();
-                // The whole row of kBlockN scores is pulled into registers at once, which frees S for the next Q K^T right
-                // away; the row is then turned into probabilities 32 columns at a time.
-                constexpr int kQuarters = kBlockN / 32;
-                uint32_t srow[kQuarters][32];
+                constexpr int kHalves = kBlockN / 32;
+                uint32_t srow[kHalves][32];
 #pragma unroll
-                for (int q = 0; q < kQuarters; ++q) tmem_ld32(s_tmem + 32 * q, srow[q]);
+                for (int q = 0; q < kHalves; ++q) tmem_ld32(s_tmem + 32 * q, srow[q]);
                 tc_wait_ld();
-                TRACE_END(1);
-                tc_fence_before();
-                mbar_arrive(&sh.s_empty[t]);
-                bool o_ready = (j == 0);  // P V of the previous key tile complete: O stable, P buffer free
                 // Row max over all scores first: independent 3-input chains of 16 scores keep the ALU pipe fed, and the
                 // rare rescale is decided once per key tile, so the exponentials below are one straight-line block.
                 float t_max = -INFINITY;
 #pragma unroll
-                for (int c = 0; c < 2 * kQuarters; ++c) {
+                for (int c = 0; c < 2 * kHalves; ++c) {
                     const uint32_t *e = &srow[c >> 1][(c & 1) * 16];
                     float m = max3(__uint_as_float(e[0]), __uint_as_float(e[1]), __uint_as_float(e[2]));
 #pragma unroll
@@ -791,30 +846,27 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                 }
                 t_max *= scale_log2;
                 const bool need = t_max > m_ref + kRescaleThreshold;  // always true on the first key tile (m_ref = -inf)
-                if (__any_sync(0xffffffffu, need)) {
+                if (__any_sync(0xffffffffu, need || !ok)) {
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) break;
                     float alpha = 1.0f;
                     if (need) {
                         alpha = (m_ref == -INFINITY) ? 0.0f : fast_exp2(m_ref - t_max);
                         m_ref = t_max;
                         l *= alpha;
                     }
-                    if (j > 0) {  // rescale what earlier key tiles accumulated
-                        ok = mbar_wait(&sh.o_done[t], (step + j - 1) & 1, sh, status, kErrODone);
-                        ok = __all_sync(0xffffffffu, ok);
-                        if (!ok) break;
-                        tc_fence_after();
-                        o_ready = true;
-                        scale_accumulator(o_tmem, alpha);
-                    }
+                    if (j > 0) scale_accumulator(o_tmem, alpha);  // rescale what earlier key tiles accumulated
                 }
                 // p = 2^(s * scale*log2e - m_ref), two scores per instruction; a share of the pairs takes the polynomial
                 // route so that the special-function unit and the FMA pipe split the exponentials.
                 const f32x2_t scale2 = pack_f32x2(scale_log2, scale_log2), neg_m2 = pack_f32x2(-m_ref, -m_ref);
                 f32x2_t sum2 = pack_f32x2(0.0f, 0.0f);
-                auto quarter = [&](const uint32_t(&a)[32], uint32_t(&pk)[16]) {
+#pragma unroll
+                for (int q = 0; q < kHalves; ++q) {
+                    uint32_t pk[16];
 #pragma unroll
                     for (int pair = 0; pair < 16; ++pair) {
-                        const f32x2_t x2 = fma_f32x2(pack_f32x2(__uint_as_float(a[2 * pair]), __uint_as_float(a[2 * pair + 1])), scale2, neg_m2);
+                        const f32x2_t x2 = fma_f32x2(pack_f32x2(__uint_as_float(srow[q][2 * pair]), __uint_as_float(srow[q][2 * pair + 1])), scale2, neg_m2);
                         float x0, x1, p0, p1;
                         unpack_f32x2(x2, x0, x1);
                         if ((kPolyPairs >> pair) & 1u) {
@@ -826,88 +878,60 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                         sum2 = add_f32x2(sum2, pack_f32x2(p0, p1));
                         pk[pair] = pack2<kBF16>(p0, p1);
                     }
-                };
-                {
-                    uint32_t pk[16];
-                    quarter(srow[0], pk);
-                    if (!o_ready) {  // the P buffer is free once P V of the previous key tile has completed
-                        TRACE_BEGIN();
-                        ok = mbar_wait(&sh.o_done[t], (step + j - 1) & 1, sh, status, kErrODone);
-                        TRACE_END(2);
-                        ok = __all_sync(0xffffffffu, ok);
-                        if (!ok) break;
-                        tc_fence_after();
-                    }
-                    tmem_st16(p_tmem, pk);  // 32 keys -> 16 columns of 16-bit pairs
-                }
-#pragma unroll
-                for (int q = 1; q < kQuarters; ++q) {
-                    uint32_t pk[16];
-                    quarter(srow[q], pk);
-                    tmem_st16(p_tmem + 16 * q, pk);
+                    tmem_st16(s_tmem + 16 * q, pk);  // 32 keys -> 16 columns of 16-bit pairs
                 }
                 {
                     float s_lo, s_hi;
                     unpack_f32x2(sum2, s_lo, s_hi);
                     l += s_lo + s_hi;
                 }
-                if (!ok) break;
-                TRACE_BEGIN();
                 tc_wait_st();
-                TRACE_END(3);
                 tc_fence_before();
                 mbar_arrive(&sh.p_full[t]);
-                TRACE_STAMP(10, step + j == 64);
             }
 
-            TRACE_BEGIN();
             if (ok) {
-                ok = mbar_wait(&sh.o_done[t], (step + n_kv - 1) & 1, sh, status, kErrODone);
+                ok = mbar_wait(&sh.o_done[t], o_phase, sh, status, kErrODone);
+                o_phase ^= 1u;
                 ok = __all_sync(0xffffffffu, ok);
             }
-            TRACE_END(6);
-            TRACE_BEGIN();
             if (ok) {
                 tc_fence_after();
-                uint32_t o[2][32];
-                tmem_ld32(o_tmem + 0, o[0]);
-                tmem_ld32(o_tmem + 32, o[1]);
-                tc_wait_ld();  // O is in registers: the next item's first P V may overwrite the accumulator
-                if (row < w.q_hi) {
-                    const float inv = 1.0f / l;
-                    // The row's 64 outputs as 32 packed words, written with 32-byte stores where the address allows it:
-                    // a warp's store then covers whole 32-byte sectors of its 32 rows instead of halves.
-                    uint32_t pk[32];
+                const int row = w.q_row0 + t * kBlockM + r;
+                const float inv = 1.0f / l;
+                T *dst_row = reinterpret_cast<T *>(out_ptr) + (int64_t)w.kpart * part_o + (int64_t)(row - q_begin) * o_rs + (int64_t)w.head * kHeadDim;
 #pragma unroll
-                    for (int c = 0; c < 2; ++c)
+                for (int c = 0; c < 2; ++c) {
+                    uint32_t o[32], pk[16];
+                    tmem_ld32(o_tmem + 32 * c, o);
+                    tc_wait_ld();  // the next item's first P V, which overwrites the accumulator, waits for this group's next P
+                    if (row < w.q_hi) {
+                        // The row's outputs as packed words, written with 32-byte stores where the address allows it: a warp's
+                        // store then covers whole 32-byte sectors of its 32 rows instead of halves.
 #pragma unroll
                         for (int i = 0; i < 32; i += 2)
-                            pk[c * 16 + i / 2] = pack2<kBF16>(__uint_as_float(o[c][i]) * inv, __uint_as_float(o[c][i + 1]) * inv);
-                    T *dst_row = reinterpret_cast<T *>(out_ptr) + (int64_t)w.kpart * part_o + (int64_t)(row - q_begin) * o_rs + (int64_t)w.head * kHeadDim;
-                    if ((reinterpret_cast<uintptr_t>(dst_row) & 31) == 0) {
+                            pk[i / 2] = pack2<kBF16>(__uint_as_float(o[i]) * inv, __uint_as_float(o[i + 1]) * inv);
+                        if ((reinterpret_cast<uintptr_t>(dst_row) & 31) == 0) {
 #pragma unroll
-                        for (int i = 0; i < 32; i += 8)
-                            asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst_row + 2 * i),
-                                         "r"(pk[i]), "r"(pk[i + 1]), "r"(pk[i + 2]), "r"(pk[i + 3]), "r"(pk[i + 4]), "r"(pk[i + 5]),
-                                         "r"(pk[i + 6]), "r"(pk[i + 7])
-                                         : "memory");
-                    } else {
-                        uint4 *dst = reinterpret_cast<uint4 *>(dst_row);
+                            for (int i = 0; i < 16; i += 8)
+                                asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst_row + 32 * c + 2 * i),
+                                             "r"(pk[i]), "r"(pk[i + 1]), "r"(pk[i + 2]), "r"(pk[i + 3]), "r"(pk[i + 4]), "r"(pk[i + 5]),
+                                             "r"(pk[i + 6]), "r"(pk[i + 7])
+                                             : "memory");
+                        } else {
+                            uint4 *dst = reinterpret_cast<uint4 *>(dst_row + 32 * c);
 #pragma unroll
-                        for (int i = 0; i < 32; i += 4) dst[i / 4] = make_uint4(pk[i], pk[i + 1], pk[i + 2], pk[i + 3]);
+                            for (int i = 0; i < 16; i += 4) dst[i / 4] = make_uint4(pk[i], pk[i + 1], pk[i + 2], pk[i + 3]);
+                        }
                     }
-                    if (lse) lse[(int64_t)w.kpart * part_l + (int64_t)w.head * (q_end - q_begin) + (row - q_begin)] = (m_ref + log2f(l)) * kLn2;
+                    __syncwarp();
                 }
+                tc_fence_before();  // the accumulator has been read; ordered before the next arrival on p_full
+                if (lse && row < w.q_hi)
+                    lse[(int64_t)w.kpart * part_l + (int64_t)w.head * (q_end - q_begin) + (row - q_begin)] = (m_ref + log2f(l)) * kLn2;
             }
-            TRACE_END(7);
-            step += n_kv;
         }
-#ifdef COME_ATTN_TRACE
-        tr_acc[4] = clock64() - tr_start;
-#endif
-        TRACE_FLUSH();
     }
-
     // ===== common exit ==========================================================================================
     tc_fence_before();
     __syncthreads();
@@ -917,7 +941,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     }
     if (warp == kIssuerWarp0) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(sh.tmem_base), "r"(kTmemCols) : "memory");
     }
 }
 
@@ -1057,7 +1081,21 @@ int attn_sm100_launch(const AttnArgs &a, cudaStream_t stream) {
     const size_t smem = sizeof(SharedStorage) + 1024 + (with_table ? kPrefixTableBytes : 0);
     const int64_t q_rows = a.q_end - a.q_begin;
     const int64_t span = a.q_free ? q_rows : (a.max_seqlen < q_rows ? a.max_seqlen : q_rows);  // most query rows any segment can own here
-    const int nblk_x = (int)((span + kTiles * kBlockM - 1) / (kTiles * kBlockM));
+    // Query tiles per work item: chosen on the device from the segments (0), except where the caller plans launches by
+    // their items (q_free: three tiles, see plan_tail_split) and where a launch has more segments than the table holds.
+    int sms = sm_count();
+    if (t_cta_limit > 0 && t_cta_limit < sms) sms = t_cta_limit;
+    const int64_t most_tiles = (span + kBlockM - 1) / kBlockM;  // of one segment
+    int tiles = a.q_free ? 3 : a.nseg > kMaxPrefixSegs ? kTiles : 0;
+    if (tiles == 0 && most_tiles * a.nseg * a.H <= sms) {
+        tiles = 1;
+    } else if (tiles == 0 && a.nseg == 1 && a.max_seqlen_dev == nullptr) {
+        HeightSums hs = {};
+        hs.add((int)most_tiles);
+        tiles = hs.best(a.H, sms);
+    }
+    const int height = tiles ? tiles : 1;
+    const int nblk_x = (int)((span + height * kBlockM - 1) / (height * kBlockM));
     const int k_parts = a.k_parts > 1 ? a.k_parts : 1;
     if (k_parts > 1) {
         // shares of the key tiles of every item: one segment whose keys all query rows attend to; no share may be empty
@@ -1074,8 +1112,6 @@ int attn_sm100_launch(const AttnArgs &a, cudaStream_t stream) {
         set_error("come_attn_varlen_fwd: %lld work items do not fit 32 bits", (long long)items);
         return COME_ERR_ARG;
     }
-    int sms = sm_count();
-    if (t_cta_limit > 0 && t_cta_limit < sms) sms = t_cta_limit;
     const unsigned grid = (unsigned)(items < sms ? items : sms);  // persistent: one CTA per SM walks the items
     const float scale_log2 = a.scale * kLog2e;
     const float inv_scale = 1.0f / a.scale;
@@ -1083,7 +1119,7 @@ int attn_sm100_launch(const AttnArgs &a, cudaStream_t stream) {
     do {                                                                                                                       \
         if ((rc = ensure_smem_optin(attn_fwd_sm100_kernel<BF16, PREFIX>, SLOT, smem)) != COME_OK) return rc;                    \
         attn_fwd_sm100_kernel<BF16, PREFIX><<<grid, kThreads, smem, stream>>>(mq, mk, mv, a.bias, a.cu, scale_log2, inv_scale, a.out, \
-                                                                              a.o_rs, a.lse, (int)a.q_begin, (int)a.q_end, nblk_x,   \
+                                                                              a.o_rs, a.lse, (int)a.q_begin, (int)a.q_end, tiles, (int)span, \
                                                                               a.nseg, a.H, a.max_seqlen_dev, status, (int)a.total,   \
                                                                               a.q_free ? 1 : 0, k_parts, (long long)a.part_o,        \
                                                                               (long long)a.part_l);                                  \
@@ -1108,12 +1144,3 @@ extern "C" int come_selftest_bounded_wait(int64_t ticks, int64_t *waited_dev, vo
     come::selftest_wait_kernel<<<1, 32, 0, (cudaStream_t)stream>>>((long long)ticks, status, (long long *)waited_dev);
     return come::check_launch("come_selftest_bounded_wait");
 }
-
-#ifdef COME_ATTN_TRACE
-// Development builds only: copies the per-warp wait counters of the last attention launch to host memory.
-extern "C" int come_debug_attn_trace(unsigned long long *host_out, int n_words) {
-    const size_t bytes = sizeof(unsigned long long) * (size_t)n_words;
-    if (bytes > sizeof(come::g_attn_trace)) return COME_ERR_ARG;
-    return cudaMemcpyFromSymbol(host_out, come::g_attn_trace, bytes) == cudaSuccess ? COME_OK : COME_ERR_CUDA;
-}
-#endif

@@ -283,6 +283,33 @@ def test_device_side_longest_segment(backend):
     _check_status()
 
 
+@pytest.mark.parametrize("kind", ["bf16", "f16"])
+@pytest.mark.parametrize("lengths", [[897], [1, 128, 129, 256, 257, 384, 385, 511, 512, 513], [60 + 31 * i for i in range(17)]])
+def test_item_heights(backend, kind, lengths):
+    """The kernel picks one to four query tiles per work item from the segments and the number of CTAs (on the host for one
+    segment, on the device without and with the per-segment table).  Every number of CTAs gives the same bits, whatever the
+    height, and the oracle's values."""
+    from come_b200 import flash_attn_fwd_cuda as fa
+    backend(fa.BACKEND_TCGEN05)
+    rng = np.random.default_rng(len(lengths))
+    P, H, D = sum(lengths), 2, 64
+    qkv = to_dev(gi.round_kind(rng.standard_normal((P, 3, H, D), dtype=np.float32), kind), kind)
+    bias = to_dev(gi.round_kind(np.log(np.where(rng.random(P) < 0.3, 9.0, 1.0)).astype(np.float32), kind), kind)
+    cu = torch.tensor(np.concatenate([[0], np.cumsum(lengths)]), dtype=torch.int32, device="cuda")
+    q, k, v = qkv[:, 0], qkv[:, 1], qkv[:, 2]
+    first = None
+    for ctas in (0, 1, 2, 3, 4, 5, 6, 8, 10, 14, 20, 40):
+        with fa.cta_limit(ctas):
+            got = fa.varlen_fwd_rows(q, k, v, cu, max(lengths), bias, D ** -0.5, 0)
+        first = got if first is None else first
+        assert torch.equal(got[0], first[0]) and torch.equal(got[1], first[1])
+    want, want_lse = clib.attention_bias(to_np(qkv), to_np(bias), cu.cpu().numpy(), D ** -0.5)
+    # outputs below 4 rounded to 8 (bfloat16) or 11 bits, probabilities rounded alike: the file's bar
+    assert np.abs(to_np(first[0]) - want).max() <= 2e-2
+    np.testing.assert_allclose(first[1].cpu().numpy(), want_lse, atol=1e-2, rtol=1e-3)
+    _check_status()
+
+
 @pytest.mark.parametrize("nseg", [15, 16, 1500, 2048, 2100])
 def test_many_short_segments(backend, nseg):
     """Thousands of short segments: around the size of the kernel's shared-memory table of per-segment query-block counts
