@@ -1,6 +1,8 @@
 """Small helpers shared by the host-side modules: dtype codes, stream and pointer access."""
 from __future__ import annotations
 
+import contextlib
+
 import torch
 
 from . import _lib
@@ -25,4 +27,17 @@ def ptr(t):
 
 
 def stream_ptr(device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    """Handle of the device's current stream (the bare handle: building a ``torch.cuda.Stream`` on every launch costs more
+    than the rest of a small launch's arguments)."""
+    index = device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
+
+
+_SAME_DEVICE = contextlib.nullcontext()
+
+
+def on_device(device):
+    """Context in which ``device`` is the current CUDA device; nothing to enter or leave when it already is."""
+    if device.index is None or device.index == torch.cuda.current_device():
+        return _SAME_DEVICE
+    return torch.cuda.device(device)

@@ -63,7 +63,7 @@ def residual_layernorm(x: torch.Tensor, branch: Optional[torch.Tensor], scale: O
     ``branch`` None: the norm of ``x`` alone; ``scale`` None: no LayerScale; ``norm`` None: the update alone.
     Returns ``(x_out, normed)``; ``x_out`` is ``x`` itself when there is no branch and None when ``store_stream`` is off."""
     from . import _lib
-    from ._torch_util import dtype_code, ptr, require_cuda, stream_ptr
+    from ._torch_util import dtype_code, on_device, ptr, require_cuda, stream_ptr
     require_cuda(x, "x")
     if x.dim() != 2 or not x.is_contiguous():
         raise ValueError(f"x must be a contiguous [rows, C] tensor, got {tuple(x.shape)}")
@@ -89,7 +89,7 @@ def residual_layernorm(x: torch.Tensor, branch: Optional[torch.Tensor], scale: O
         raise ValueError("nothing to compute: neither a branch nor a norm")
     x_out = torch.empty_like(x) if (branch is not None and store_stream) else None
     normed = torch.empty_like(x) if norm is not None else None
-    with torch.cuda.device(dev):
+    with on_device(dev):
         _lib.check(_lib.lib().come_residual_layernorm(ptr(x), ptr(branch), ptr(scale), rows, Cc, dtype_code(dt, "x"), ptr(gamma),
                                                       ptr(beta), eps, ptr(x_out), ptr(normed), stream_ptr(dev)))
     return (x if branch is None else x_out), normed

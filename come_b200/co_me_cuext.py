@@ -13,7 +13,7 @@ import ctypes as C
 import torch
 
 from . import _lib
-from ._torch_util import dtype_code, ptr, require_cuda, stream_ptr
+from ._torch_util import dtype_code, on_device, ptr, require_cuda, stream_ptr
 
 __all__ = ["co_me_token_merge_cuda", "co_me_token_split_cuda", "merge_plan_raw"]
 
@@ -21,17 +21,18 @@ __all__ = ["co_me_token_merge_cuda", "co_me_token_split_cuda", "merge_plan_raw"]
 def merge_plan_raw(mask_u8: torch.Tensor, layout: _lib.Layout, tokens_per_frame: int):
     """Run the index plan of a merge.  Returns device tensors
     ``(group_prefix i32 [F,M], offsets i32 [F+1], rev_id i64 [F*N], weight f32 [F*N] (first P valid), seg_max i32 [1])``.
+    ``offsets`` and ``seg_max`` are neighbours in one buffer, so that one copy brings both lengths to the host.
     """
     frames, M = mask_u8.shape
     dev = mask_u8.device
     group_prefix = torch.empty((frames, M), dtype=torch.int32, device=dev)
-    offsets = torch.empty((frames + 1,), dtype=torch.int32, device=dev)
+    lengths = torch.empty((frames + 2,), dtype=torch.int32, device=dev)
+    offsets, seg_max = lengths[:-1], lengths[-1:]
     rev = torch.empty((frames * tokens_per_frame,), dtype=torch.int64, device=dev)
     weight = torch.empty((max(frames * tokens_per_frame, 1),), dtype=torch.float32, device=dev)
-    seg_max = torch.empty((1,), dtype=torch.int32, device=dev)
     ws_bytes = _lib.lib().come_merge_plan_workspace_bytes(frames)
     ws = torch.empty((ws_bytes,), dtype=torch.uint8, device=dev)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         _lib.check(_lib.lib().come_merge_plan(ptr(mask_u8), frames, C.byref(layout), ptr(group_prefix), ptr(offsets),
                                               ptr(rev), ptr(weight), ptr(seg_max), ptr(ws), ws_bytes, stream_ptr(dev)))
     return group_prefix, offsets, rev, weight, seg_max
@@ -71,7 +72,7 @@ def co_me_token_merge_cuda(tokens: torch.Tensor, start_index: int, group_size: i
     # mask.sum() at the same point, kernel_token_merge.cu:265).
     P = int(offsets[-1].item()) if B > 0 else 0
     out = torch.empty((P, Cc), dtype=tokens_c.dtype, device=tokens_c.device)
-    with torch.cuda.device(tokens_c.device):
+    with on_device(tokens_c.device):
         _lib.check(_lib.lib().come_merge(ptr(tokens_c), code, B, Cc, C.byref(layout), ptr(mask_u8), ptr(group_prefix),
                                          ptr(offsets), ptr(out), stream_ptr(tokens_c.device)))
     return out, offsets, rev, weight[:P]
@@ -92,7 +93,7 @@ def co_me_token_split_cuda(merged_flat: torch.Tensor, rev_id: torch.Tensor, C_: 
     total = rev_c.numel()
     code = dtype_code(merged_c.dtype, "merged_flat")
     out = torch.empty((total, C_), dtype=merged_c.dtype, device=merged_c.device)
-    with torch.cuda.device(merged_c.device):
+    with on_device(merged_c.device):
         _lib.check(_lib.lib().come_unmerge(ptr(merged_c), ptr(rev_c), total, C_, code, ptr(out),
                                            stream_ptr(merged_c.device)))
     return out

@@ -46,9 +46,10 @@ class _VarlenQKVPacked(torch.autograd.Function):
                 window_size, softcap, alibi_slopes, return_softmax, max_seqlen_dev=None):
         if softmax_scale is None:
             softmax_scale = qkv.shape[-1] ** (-0.5)
-        q, k, v = qkv[:, 0].detach(), qkv[:, 1].detach(), qkv[:, 2].detach()
+        q, k, v = qkv.detach().unbind(1)[:3]
         head_size_og = q.size(2)
-        q, k, v = (_pad_head(x, head_size_og) for x in (q, k, v))
+        if head_size_og % 8 != 0:
+            q, k, v = (_pad_head(x, head_size_og) for x in (q, k, v))
         common = (dropout_p, softmax_scale, False, causal, window_size[0], window_size[1], softcap,
                   return_softmax and dropout_p > 0, None)
         if has_bias:
@@ -60,7 +61,7 @@ class _VarlenQKVPacked(torch.autograd.Function):
                 q, k, v, None, cu_seqlens, cu_seqlens, None, None, None, alibi_slopes, max_seqlen, max_seqlen, *common,
                 max_seqlen_dev=max_seqlen_dev)
         ctx.mark_non_differentiable(softmax_lse, S_dmask, rng_state)
-        out = out_padded[..., :head_size_og]
+        out = out_padded if out_padded.shape[-1] == head_size_og else out_padded[..., :head_size_og]
         return out if not return_softmax else (out, softmax_lse, S_dmask)
 
     @staticmethod

@@ -13,7 +13,7 @@ import threading
 import torch
 
 from . import _lib
-from ._torch_util import dtype_code, ptr, stream_ptr
+from ._torch_util import dtype_code, on_device, ptr, stream_ptr
 
 __all__ = ["varlen_fwd", "varlen_fwd_w_perkey_bias", "varlen_fwd_rows", "cross_fwd", "cross_fwd_balanced", "plan_tail_split",
            "combine"]
@@ -154,7 +154,7 @@ def _impl(q, k, v, out_, cu_seqlens_q, cu_seqlens_k, seqused_k, leftpad_k, block
         return t if t.stride(1) == head_size else t.contiguous()
 
     q, k, v = head_packed(q), head_packed(k), head_packed(v)
-    with torch.cuda.device(q.device):
+    with on_device(q.device):
         if max_seqlen_dev is None:
             _lib.check(_lib.lib().come_attn_varlen_fwd(
                 ptr(q), ptr(k), ptr(v), dtype_code(q.dtype), total_q, num_heads, head_size, q.stride(0), k.stride(0),
@@ -223,7 +223,7 @@ def varlen_fwd_rows(q_rows, k, v, cu_seqlens, max_seqlen, perkey_bias, softmax_s
         raise RuntimeError("perkey_bias must be a contiguous (total,) tensor of the q/k/v dtype")
     out = out_ if out_ is not None else torch.empty((rows, num_heads, head_size), dtype=q_rows.dtype, device=q_rows.device)
     lse = torch.empty((num_heads, rows), dtype=torch.float32, device=q_rows.device)
-    with torch.cuda.device(q_rows.device):
+    with on_device(q_rows.device):
         _lib.check(_lib.lib().come_attn_varlen_fwd_rows(
             ptr(q_rows), ptr(k), ptr(v), dtype_code(q_rows.dtype), total, int(row_begin), rows, num_heads, head_size,
             q_rows.stride(0), k.stride(0), v.stride(0), ptr(perkey_bias), ptr(cu_seqlens), cu_seqlens.numel() - 1,
@@ -257,7 +257,7 @@ def cross_fwd(q_rows, k, v, perkey_bias, softmax_scale, out_=None):
         raise RuntimeError("perkey_bias must be a contiguous (kv_rows,) tensor of the q/k/v dtype")
     out = out_ if out_ is not None else torch.empty((rows, num_heads, head_size), dtype=q_rows.dtype, device=q_rows.device)
     lse = torch.empty((num_heads, rows), dtype=torch.float32, device=q_rows.device)
-    with torch.cuda.device(q_rows.device):
+    with on_device(q_rows.device):
         _lib.check(_lib.lib().come_attn_cross_fwd(
             ptr(q_rows), ptr(k), ptr(v), dtype_code(q_rows.dtype), rows, kv_rows, num_heads, head_size, q_rows.stride(0),
             k.stride(0), v.stride(0), ptr(perkey_bias), float(softmax_scale), ptr(out), out.stride(0), ptr(lse), _backend,
@@ -309,7 +309,7 @@ def cross_fwd_balanced(q_rows, k, v, perkey_bias, softmax_scale, out_=None):
     out_parts = torch.empty((parts, n_tail, num_heads, head_size), dtype=q_rows.dtype, device=q_rows.device)
     lse_parts = torch.empty((parts, num_heads, n_tail), dtype=torch.float32, device=q_rows.device)
     lse_tail = torch.empty((num_heads, n_tail), dtype=torch.float32, device=q_rows.device)
-    with torch.cuda.device(q_rows.device):
+    with on_device(q_rows.device):
         lib, st = _lib.lib(), stream_ptr(q_rows.device)
         rc = lib.come_attn_cross_fwd_parts(
             ptr(tail), ptr(k), ptr(v), dtype_code(q_rows.dtype), n_tail, k.shape[0], num_heads, head_size, tail.stride(0),
@@ -337,7 +337,7 @@ def combine(out_a, lse_a, out_b, lse_b, out_=None, lse_out=None):
         raise RuntimeError("combine needs contiguous results")
     out = out_ if out_ is not None else torch.empty_like(out_a)
     lse = lse_out if lse_out is not None else torch.empty_like(lse_a)
-    with torch.cuda.device(out_a.device):
+    with on_device(out_a.device):
         _lib.check(_lib.lib().come_attn_combine(ptr(out_a), ptr(lse_a), ptr(out_b), ptr(lse_b), dtype_code(out_a.dtype), rows,
                                                 num_heads, head_size, ptr(out), ptr(lse), stream_ptr(out_a.device)))
     return [out, lse]

@@ -12,7 +12,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from ._torch_util import dtype_code, ptr, require_cuda, stream_ptr
+from ._torch_util import dtype_code, on_device, ptr, require_cuda, stream_ptr
 
 __all__ = ["RotaryPositionEmbedding2D", "prepare_packed_self_attention_qkv"]
 
@@ -115,7 +115,7 @@ def prepare_packed_self_attention_qkv(qkv: torch.Tensor, q_norm, k_norm, rope, p
             raise RuntimeError(f"weight must be [{P}], got {tuple(weight.shape)}")
         weight = weight.to(torch.float32).contiguous()
         bias = torch.empty(P, dtype=run_dtype, device=dev)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         _lib.check(_lib.lib().come_qkv_prepare(
             ptr(qkv), code, P, H, D, ptr(qg), ptr(qb), ptr(kg), ptr(kb), q_eps, ptr(pos), ptr(cos), ptr(sin), rows,
             ptr(weight), ptr(bias), stream_ptr(dev)))

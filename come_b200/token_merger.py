@@ -22,7 +22,7 @@ from typing import Any, Callable, Optional, Tuple
 import torch
 
 from . import _lib, co_me_cuext
-from ._torch_util import dtype_code, ptr, require_cuda, stream_ptr
+from ._torch_util import dtype_code, on_device, ptr, require_cuda, stream_ptr
 
 __all__ = [
     "JaggedTokens", "MergePlan", "func_token_merge", "func_token_split", "func_token_merge_2d", "select_windows",
@@ -80,7 +80,7 @@ class JaggedTokens:
             new_tokens = torch.empty(1, P_old + M * T, Cc, device=dev, dtype=tokens.dtype)
             new_weight = torch.empty(P_old + M * T, device=dev, dtype=torch.float32)
             new_offset = torch.empty_like(offset)
-            with torch.cuda.device(dev):
+            with on_device(dev):
                 _lib.check(_lib.lib().come_suffix_add(ptr(tokens), ptr(weight), ptr(offset), M, P_old, Cc,
                                                       dtype_code(tokens.dtype, "tokens"), ptr(suffix), T, ptr(new_tokens),
                                                       ptr(new_weight), ptr(new_offset), stream_ptr(dev)))
@@ -120,7 +120,7 @@ class JaggedTokens:
             new_weight = torch.empty(P_new, device=tdev, dtype=torch.float32)
             new_offset = torch.empty_like(offset)
             suffix = torch.empty(M, T, Cc, device=tdev, dtype=tokens.dtype)
-            with torch.cuda.device(tdev):
+            with on_device(tdev):
                 _lib.check(_lib.lib().come_suffix_split(ptr(tokens), ptr(weight), ptr(offset), M, P_old, Cc,
                                                         dtype_code(tokens.dtype, "tokens"), T, ptr(new_tokens),
                                                         ptr(new_weight), ptr(new_offset), ptr(suffix), stream_ptr(tdev)))
@@ -206,7 +206,8 @@ class MergePlan:
             self._mask_u8, layout, self.tokens_per_frame)
         self.seg_max = seg_max  # [1] int32 on the device: the longest frame after merging
         if self.frames > 0:
-            host = torch.stack([self.offsets_i32[-1], seg_max[0]]).tolist()  # the single synchronising read
+            # the single synchronising read: the last offset and the longest frame, which follows it in memory
+            host = self.offsets_i32.as_strided((2,), (1,), self.offsets_i32.storage_offset() + self.frames).tolist()
             self.total, self.max_seqlen = int(host[0]), int(host[1])
         else:
             self.total, self.max_seqlen = 0, 0
@@ -247,7 +248,7 @@ class MergePlan:
         truncating it (``src/accelerate/vggt/fused.py:113-129``).  2-D layouts only."""
         if self._positions is None:
             pos = torch.empty(self.total, 2, dtype=torch.int64, device=self.mask.device)
-            with torch.cuda.device(self.mask.device):
+            with on_device(self.mask.device):
                 _lib.check(_lib.lib().come_packed_positions(ptr(self._mask_u8), ptr(self.rev_id), self.frames,
                                                             C.byref(self.layout), ptr(pos),
                                                             stream_ptr(self.mask.device)))
@@ -262,7 +263,7 @@ class MergePlan:
             raise ValueError(f"Expected tokens [{self.frames}, {self.tokens_per_frame}, C], got {tuple(tokens.shape)}")
         tokens = tokens.contiguous()
         out = torch.empty((self.total, tokens.shape[2]), dtype=tokens.dtype, device=tokens.device)
-        with torch.cuda.device(tokens.device):
+        with on_device(tokens.device):
             _lib.check(_lib.lib().come_merge(ptr(tokens), dtype_code(tokens.dtype, "tokens"), self.frames,
                                              tokens.shape[2], C.byref(self.layout), ptr(self._mask_u8),
                                              ptr(self.group_prefix), ptr(self.offsets_i32), ptr(out),
@@ -284,7 +285,7 @@ class MergePlan:
         w = (norm.weight if norm.weight is not None else torch.ones(Cc, device=dev)).detach().to(device=dev, dtype=dt).contiguous()
         b = (norm.bias if norm.bias is not None else torch.zeros(Cc, device=dev)).detach().to(device=dev, dtype=dt).contiguous()
         out = torch.empty((self.total, Cc), dtype=dt, device=dev)
-        with torch.cuda.device(dev):
+        with on_device(dev):
             _lib.check(_lib.lib().come_merge_layernorm(ptr(tokens), dtype_code(dt, "tokens"), self.frames, Cc,
                                                        C.byref(self.layout), ptr(w), ptr(b), float(norm.eps),
                                                        ptr(self._mask_u8), ptr(self.group_prefix), ptr(self.offsets_i32),
@@ -316,7 +317,7 @@ class MergePlan:
             out = torch.empty_like(residual)
         elif out.shape != residual.shape or out.dtype != residual.dtype or not out.is_contiguous():
             raise ValueError("out must be contiguous and match residual")
-        with torch.cuda.device(merged.device):
+        with on_device(merged.device):
             _lib.check(_lib.lib().come_unmerge_residual(ptr(merged), ptr(self.rev_id), rows, Cc,
                                                         dtype_code(merged.dtype, "merged"), ptr(residual),
                                                         ptr(None if scale is None else scale.contiguous()), ptr(out),
@@ -339,7 +340,7 @@ class MergePlan:
         out = torch.empty((rows, width), dtype=first.dtype, device=first.device)
         code = dtype_code(first.dtype, "merged")
         col = 0
-        with torch.cuda.device(first.device):
+        with on_device(first.device):
             for m in merged:
                 m = m.contiguous()
                 dst = out.data_ptr() + col * out.element_size()
@@ -427,12 +428,12 @@ def select_windows(confidence: torch.Tensor, B: int, S: int, H: int, W: int, gro
     mask = torch.empty((B * S, M), dtype=torch.bool, device=conf.device)
     if ratios is not None:
         ratios = ratios.contiguous()
-        with torch.cuda.device(conf.device):
+        with on_device(conf.device):
             _lib.check(_lib.lib().come_select_windows_ratios(
                 ptr(conf), dtype_code(conf.dtype, "confidence"), B, S, H, W, group_h, group_w, ptr(ratios),
                 _lib.COME_SCOPE_BATCH if scope == "batch" else _lib.COME_SCOPE_FRAME, ptr(mask), stream_ptr(conf.device)))
         return mask
-    with torch.cuda.device(conf.device):
+    with on_device(conf.device):
         _lib.check(_lib.lib().come_select_windows(
             ptr(conf), dtype_code(conf.dtype, "confidence"), B, S, H, W, group_h, group_w, float(threshold),
             _SELECT_MODES[mode],
