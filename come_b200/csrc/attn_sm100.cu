@@ -191,18 +191,6 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
         : "r"(taddr)
         : "memory");
 }
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
-        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
-          "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]),
-          "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]),
-          "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
-        : "memory");
-}
-
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
@@ -343,14 +331,23 @@ __device__ __forceinline__ int segment_tiles(int seg, const int *__restrict__ cu
 }
 
 // Query tiles per work item.  A key step of an item costs less than in proportion to its tiles (the tiles share the SM's
-// units but each is a latency chain: 0.76 / 0.88 / 1.15 / 1.35 us with 1 / 2 / 3 / 4 tiles, 80,672 keys), so four tiles are
+// units but each is a latency chain: 0.79 / 0.90 / 1.06 / 1.29 us with 1 / 2 / 3 / 4 tiles, 6456 keys), so four tiles are
 // best where there are many items; but the items are dealt to the CTAs in rounds, and with few of them the height that
 // fills its last round wins: 6456 tokens x 16 heads take 215 us with 3 (272 items, 2 rounds) and 260 with 4 (208 items, also
 // 2 rounds); 3228 tokens 59 and 68 us; 2 segments of ~450 tokens 12.0 us with 1 and 16.8 with 4; 4 x 807 tokens 24 us with
-// 4 and 37 with 3.  The choice is the height with the least (rounds of items over the CTAs) x (mean cost of an item).  The
+// 4 and 37 with 3.  The choice is the height with the least (full rounds of items over the CTAs) x (mean cost of an item) + the last
+// round, whose items are split into lower ones where the CTAs suffice for that (tail_height): 24,576 tokens x 16 heads are
+// 768 items = 5 rounds + 28 items of four tiles, which run as 112 items of one (3.02 -> 2.87 ms); 80,672 tokens are 17
+// rounds + 12 items (30.6 -> 29.7 ms).  The
 // segments of a launch are known exactly on the device only, so every CTA makes the same choice from them (about 1 us of
 // the launch); the host makes it for one segment, and where every query tile gets a CTA of its own.
-__host__ __device__ __forceinline__ int step_cost(int n) { return n <= 0 ? 0 : n == 1 ? 64 : n == 2 ? 73 : n == 3 ? 96 : 113; }
+__host__ __device__ __forceinline__ int step_cost(int n) { return n <= 0 ? 0 : n == 1 ? 70 : n == 2 ? 80 : n == 3 ? 96 : 115; }
+// Height of the items of the last, partial round of `rest` items of `height` tiles.
+__host__ __device__ __forceinline__ int tail_height(int height, int rest, int ctas) {
+    if (height > 1 && rest * height <= ctas) return 1;
+    if (height > 2 && rest * 2 <= ctas) return 2;
+    return height;
+}
 struct HeightSums {
     int items[kTiles], cost[kTiles];  // [height - 1], of one head
     __host__ __device__ __forceinline__ void add(int n) {
@@ -372,8 +369,9 @@ struct HeightSums {
         float least = 3.0e38f;
 #pragma unroll
         for (int h = kTiles; h >= 1; --h) {
-            const int rounds = (items[h - 1] * num_heads + ctas - 1) / ctas;
-            const float t = (float)rounds * (float)cost[h - 1] / (float)(items[h - 1] > 0 ? items[h - 1] : 1);
+            const int n = items[h - 1] * num_heads, rest = n % ctas, low = tail_height(h, rest, ctas);
+            const float mean = (float)cost[h - 1] / (float)(items[h - 1] > 0 ? items[h - 1] : 1);
+            const float t = (float)(n / ctas) * mean + (rest == 0 ? 0.0f : low == h ? mean : (float)step_cost(low));
             if (t < least) {
                 least = t;
                 height = h;
@@ -383,6 +381,11 @@ struct HeightSums {
     }
 };
 
+// The items from `from` on (the last, partial round) are split into `parts` items of `tiles` query tiles.
+struct TailSplit {
+    int from, parts, tiles;
+};
+
 // Item -> (head, segment, query block).  With a prefix table (seg_prefix != nullptr) the items are exactly the query
 // blocks that exist, in (head, segment, block) order; without it every segment gets `nblk_x` slots and the surplus ones
 // are skipped as invalid.
@@ -390,12 +393,20 @@ struct HeightSums {
 // inside the segment (attention of this GPU's rows to keys gathered from other GPUs); cu may then be NULL = [0, kv_total].
 template <bool kPrefix>
 __device__ __forceinline__ WorkItem decode_item(int item, int nblk_x, int nseg, const int *__restrict__ cu, int q_begin, int q_end,
-                                                const int *seg_prefix, int kv_total, bool q_free, int tiles, int k_parts) {
+                                                const int *seg_prefix, int kv_total, bool q_free, int tiles, int k_parts,
+                                                const TailSplit &tail) {
     WorkItem w;
     int bx, seg;
     // Launches with k_parts > 1 (q_free only): consecutive items are the shares of the key tiles of one (head, block); every
     // share writes its own output and log-sum-exp, merged afterwards.  The host picks k_parts so that no share is empty.
     w.kpart = 0;
+    int sub = 0;  // position inside a split item
+    if (item >= tail.from) {
+        const int i = item - tail.from;
+        sub = i % tail.parts;
+        item = tail.from + i / tail.parts;
+    }
+    const bool split = tail.parts > 1 && item >= tail.from;
     if (k_parts > 1) {
         w.kpart = item % k_parts;
         item /= k_parts;
@@ -426,8 +437,13 @@ __device__ __forceinline__ WorkItem decode_item(int item, int nblk_x, int nseg, 
     const int q_lo = q_free ? q_begin : max(w.s0, q_begin);
     w.q_hi = q_free ? q_end : min(w.s1, q_end);
     w.q_row0 = q_lo + bx * (tiles * kBlockM);
-    w.valid = w.q_row0 < w.q_hi;
-    w.n_mt = min(tiles, (w.q_hi - w.q_row0 + kBlockM - 1) / kBlockM);  // query tiles with at least one valid row
+    int rows = min(w.q_hi - w.q_row0, tiles * kBlockM);  // of the item
+    if (split) {
+        w.q_row0 += sub * (tail.tiles * kBlockM);
+        rows = min(rows - sub * (tail.tiles * kBlockM), tail.tiles * kBlockM);
+    }
+    w.valid = rows > 0;
+    w.n_mt = (rows + kBlockM - 1) / kBlockM;  // query tiles with at least one valid row
     w.n_kv = (seg_len + kBlockN - 1) / kBlockN;
     w.ragged_tail = (seg_len % kBlockN) != 0;
     if (k_parts > 1) {
@@ -457,7 +473,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                       const __grid_constant__ CUtensorMap map_v, const void *__restrict__ bias_ptr,
                       const int *__restrict__ cu, float scale_log2, float inv_scale, void *__restrict__ out_ptr, int64_t o_rs,
                       float *__restrict__ lse, int q_begin, int q_end, int tiles, int max_rows, int nseg, int num_heads,
-                      const int *__restrict__ max_len_dev, unsigned int *__restrict__ status, int kv_total, int q_free_flag,
+                      const int *__restrict__ max_len_dev, unsigned int *__restrict__ status, int kv_total, int q_free_flag, int split_tail,
                       int k_parts, long long part_o, long long part_l) {
     using T = typename std::conditional<kBF16, __nv_bfloat16, __half>::type;
     // the declared alignment makes the base, and with it every barrier address and matrix descriptor, a link-time constant
@@ -542,7 +558,17 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         }
     }
     const int *seg_prefix = use_prefix ? prefix_table : nullptr;
-    const int total_items = (use_prefix ? prefix_table[nseg] * num_heads : nblk_x * nseg * num_heads) * k_parts;
+    int total_items = (use_prefix ? prefix_table[nseg] * num_heads : nblk_x * nseg * num_heads) * k_parts;
+    TailSplit tail{total_items, 1, tiles};
+    if (split_tail) {
+        const int rest = total_items % (int)gridDim.x;
+        tail.tiles = tail_height(tiles, rest, gridDim.x);
+        if (tail.tiles != tiles) {
+            tail.parts = (tiles + tail.tiles - 1) / tail.tiles;
+            tail.from = total_items - rest;
+            total_items = tail.from + rest * tail.parts;
+        }
+    }
     const bool has_bias = bias_ptr != nullptr;
     const bool q_free = q_free_flag != 0;
     // a key tile needs the bias step when there is a bias, or when it is the partial last tile (masking)
@@ -605,7 +631,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
             int it = 0;      // ring position, advanced once per key tile
             int q_uses = 0;  // items loaded so far (buffer and phase of q_full / q_empty)
             for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x) {
-                const WorkItem w = decode_item<kPrefix>(item, nblk_x, nseg, cu, q_begin, q_end, seg_prefix, kv_total, q_free, tiles, k_parts);
+                const WorkItem w = decode_item<kPrefix>(item, nblk_x, nseg, cu, q_begin, q_end, seg_prefix, kv_total, q_free, tiles, k_parts, tail);
                 if (!w.valid) continue;
                 if (lane == 0) {
                     // Item n uses Q buffer n & 1, free once the last tensor-core work of item n - 2 has completed: the next
@@ -696,7 +722,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                 };
                 auto next_valid = [&](int &item, Item &x) -> bool {
                     for (; item < total_items; item += gridDim.x) {
-                        const WorkItem w = decode_item<kPrefix>(item, nblk_x, nseg, cu, q_begin, q_end, seg_prefix, kv_total, q_free, tiles, k_parts);
+                        const WorkItem w = decode_item<kPrefix>(item, nblk_x, nseg, cu, q_begin, q_end, seg_prefix, kv_total, q_free, tiles, k_parts, tail);
                         if (w.valid) {
                             x = Item{w.n_mt, w.n_kv, w.ragged_tail};
                             return true;
@@ -816,7 +842,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         bool ok = true;
         uint32_t s_phase = 0, o_phase = 0;
         for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x) {
-            const WorkItem w = decode_item<kPrefix>(item, nblk_x, nseg, cu, q_begin, q_end, seg_prefix, kv_total, q_free, tiles, k_parts);
+            const WorkItem w = decode_item<kPrefix>(item, nblk_x, nseg, cu, q_begin, q_end, seg_prefix, kv_total, q_free, tiles, k_parts, tail);
             if (!w.valid || t >= w.n_mt) continue;
             const int n_kv = w.n_kv;
             float m_ref = -INFINITY, l = 0.0f;  // reference max (log2 units, scale applied) and running sum
@@ -1094,7 +1120,8 @@ int attn_sm100_launch(const AttnArgs &a, cudaStream_t stream) {
         hs.add((int)most_tiles);
         tiles = hs.best(a.H, sms);
     }
-    const int height = tiles ? tiles : 1;
+    const int split_tail = !a.q_free && a.nseg <= kMaxPrefixSegs ? 1 : 0;  // launches whose items all exist
+    const int height = tiles == 0 || split_tail ? 1 : tiles;  // of the lowest items the launch may have
     const int nblk_x = (int)((span + height * kBlockM - 1) / (height * kBlockM));
     const int k_parts = a.k_parts > 1 ? a.k_parts : 1;
     if (k_parts > 1) {
@@ -1121,7 +1148,7 @@ int attn_sm100_launch(const AttnArgs &a, cudaStream_t stream) {
         attn_fwd_sm100_kernel<BF16, PREFIX><<<grid, kThreads, smem, stream>>>(mq, mk, mv, a.bias, a.cu, scale_log2, inv_scale, a.out, \
                                                                               a.o_rs, a.lse, (int)a.q_begin, (int)a.q_end, tiles, (int)span, \
                                                                               a.nseg, a.H, a.max_seqlen_dev, status, (int)a.total,   \
-                                                                              a.q_free ? 1 : 0, k_parts, (long long)a.part_o,        \
+                                                                              a.q_free ? 1 : 0, split_tail, k_parts, (long long)a.part_o, \
                                                                               (long long)a.part_l);                                  \
     } while (0)
     if (a.dtype == COME_BF16) {
