@@ -29,9 +29,12 @@
 // at link time, one copy of the code per issuer and no vote or loop exit that depends on a wait, the nine instructions of a
 // tile and step are issued in ~190 clocks; with operands moved from ordinary registers they took ~590.
 //
-// Every wait on an mbarrier is bounded: after ~2^29 clock ticks the waiter raises the CTA's abort flag and the
-// library's device status word, every role falls through to the common exit, TMEM is released and the kernel
-// returns instead of hanging.
+// Every wait on an mbarrier is bounded: after ~2^29 clock ticks the waiter raises the CTA's abort flag and the library's
+// device status word.  From then on no role acts on data it did not wait for: the producer loads and an issuer issues
+// nothing more, and a softmax group stores an item only if the last P V of it was issued and has completed, so a row of the
+// result is either right or untouched.  Every role falls through to the common exit, where the producer waits for its own
+// loads and the issuers for their own tensor-core work (both complete by themselves; bounded all the same); then TMEM is
+// released and the kernel returns instead of hanging.
 #include "attn_sm100.cuh"
 
 #include <cuda.h>
@@ -90,6 +93,7 @@ struct SharedStorage {
     uint64_t s_full[kTiles];  // scores of a key tile complete (and, in order before them, P V of the key tile before)
     uint64_t p_full[kTiles];
     uint64_t o_done[kTiles];  // the last P V of an item complete
+    uint64_t drained;         // all tensor-core work of the CTA complete (exit path)
     uint32_t tmem_base;
     volatile uint32_t abort_flag;
     int scan_warp[kThreads / 32];
@@ -143,6 +147,16 @@ __device__ __forceinline__ bool mbar_wait_limit(uint64_t *bar, uint32_t parity, 
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, SharedStorage &sh, unsigned int *status,
                                           uint32_t code) {
     return mbar_wait_limit(bar, parity, &sh.abort_flag, status, code, kWaitTicks);
+}
+// Bounded wait of the exit path, for work of this CTA that completes by itself: it goes on after the abort flag is raised.
+__device__ __forceinline__ void mbar_drain(uint64_t *bar, uint32_t parity, unsigned int *status, uint32_t code) {
+    const long long t0 = clock64();
+    while (!mbar_try_wait(bar, parity)) {
+        if (clock64() - t0 > kWaitTicks) {
+            atomicOr(status, code);
+            return;
+        }
+    }
 }
 
 __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, int c0, int c1, int c2, uint64_t *bar) {
@@ -467,14 +481,15 @@ __device__ __forceinline__ WorkItem decode_item(int item, int nblk_x, int nseg, 
 // streams the next item's K/V (and, once the last Q K^T of the current item has completed, its Q) while the softmax
 // groups are still finishing the current one.
 // kPrefix selects the work list at compile time, so that launches with few segments carry none of the table's code.
-template <bool kBF16, bool kPrefix>
+// kSelfTest: the producer loads the key tiles before the CTA's tile `stall_tile` only, so that the waits for that tile run out.
+template <bool kBF16, bool kPrefix, bool kSelfTest = false>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                       const __grid_constant__ CUtensorMap map_v, const void *__restrict__ bias_ptr,
                       const int *__restrict__ cu, float scale_log2, float inv_scale, void *__restrict__ out_ptr, int64_t o_rs,
                       float *__restrict__ lse, int q_begin, int q_end, int tiles, int max_rows, int nseg, int num_heads,
                       const int *__restrict__ max_len_dev, unsigned int *__restrict__ status, int kv_total, int q_free_flag, int split_tail,
-                      int k_parts, long long part_o, long long part_l) {
+                      int k_parts, long long part_o, long long part_l, int stall_tile) {
     using T = typename std::conditional<kBF16, __nv_bfloat16, __half>::type;
     // the declared alignment makes the base, and with it every barrier address and matrix descriptor, a link-time constant
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -593,6 +608,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
             mbar_init(&sh.kv_empty[i], kIssuers);
         }
         mbar_init(&sh.q_slab_full, 1);
+        mbar_init(&sh.drained, kIssuers);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == kIssuerWarp0) {
@@ -628,8 +644,8 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&sh.q_slab_full);
             }
-            int it = 0;      // ring position, advanced once per key tile
-            int q_uses = 0;  // items loaded so far (buffer and phase of q_full / q_empty)
+            int it = 0;      // ring position = key tiles loaded so far
+            int q_uses = 0;  // items whose Q was loaded so far (buffer and phase of q_full / q_empty)
             for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x) {
                 const WorkItem w = decode_item<kPrefix>(item, nblk_x, nseg, cu, q_begin, q_end, seg_prefix, kv_total, q_free, tiles, k_parts, tail);
                 if (!w.valid) continue;
@@ -644,8 +660,9 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                             tma_load_3d(sh.q[b][t], &map_q, 0, w.head, w.q_row0 - q_begin + t * kBlockM, &sh.q_full[b]);
                     }
                 }
-                ++q_uses;
                 ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                ++q_uses;
                 // bias of the lane's keys, fetched one key tile ahead of its use
                 float next_bias[kBlockN / 32];
                 auto fetch_bias = [&](int j) {
@@ -658,6 +675,12 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                 fetch_bias(0);
                 for (int j = 0; j < w.n_kv && ok; ++j, ++it) {
                     const int st = it % kStages;
+                    if constexpr (kSelfTest) {
+                        if (it >= stall_tile) {  // the waits for this tile run out
+                            ok = false;
+                            break;
+                        }
+                    }
                     ok = mbar_wait(&sh.kv_empty[st], ((it / kStages) & 1) ^ 1, sh, status, kErrKvEmpty);
                     ok = __all_sync(0xffffffffu, ok);
                     if (!ok) break;
@@ -682,6 +705,12 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                     if (j + 1 < w.n_kv) fetch_bias(j + 1);
                 }
             }
+            if (lane == 0) {  // the last use of every buffer has landed before the shared memory is released
+                for (int i = max(it - kStages, 0); i < it; ++i)
+                    mbar_drain(&sh.kv_full[i % kStages], (i / kStages) & 1, status, kErrKvFull);
+                for (int n = max(q_uses - 2, 0); n < q_uses; ++n) mbar_drain(&sh.q_full[n & 1], (n >> 1) & 1, status, kErrQFull);
+            }
+            __syncwarp();
         } else if (warp < kIssuerWarp0 + kIssuers) {
             // ===== MMA issuers: query tiles first, first + kIssuers, ... ====================================
             // One copy of the code per issuer and uniform control flow, so that the operands of the tensor-core instructions
@@ -734,49 +763,57 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                 uint32_t st = 0, kv_phase = 0;  // ring stage of the current key tile; phase of kv_full for the stage after it
                 uint32_t p_phase = 0;           // bit t: phase of p_full[t]
                 uint32_t qb = 0, q_phase = 0;   // Q buffer of the current item; bit b: phase of q_full[b]
-                int items = 0;                  // items done
                 int item = blockIdx.x;
                 Item w, nx;
                 bool have = next_valid(item, w);
-                mbar_wait(&sh.q_slab_full, 0, sh, status, kErrQFull);
+                // A lane's own "no wait has given up": after a failure its elected lane issues nothing more and its waits try their
+                // barrier once.  It does not steer the key loop (that would make the operands non-uniform) except by a vote every
+                // 32 key tiles.  A branch on it in front of every wait measured 0.3 % slower.
+                bool ok = true;
+                auto wait = [&](uint64_t &bar, uint32_t parity, uint32_t code) {
+                    if (!mbar_try_wait(&bar, parity)) ok = ok && mbar_wait(&bar, parity, sh, status, code);
+                };
+                wait(sh.q_slab_full, 0, kErrQFull);
                 if (have) {  // the first scores of the first item; later items' first scores are issued with the last P V before them
-                    mbar_wait(&sh.q_full[0], 0, sh, status, kErrQFull);
-                    mbar_wait(&sh.kv_full[0], 0, sh, status, kErrKvFull);
+                    wait(sh.q_full[0], 0, kErrQFull);
+                    wait(sh.kv_full[0], 0, kErrKvFull);
                     q_phase ^= 1u;
                     __syncwarp();
                     tc_fence_after();
-                    if (elect_one()) {
+                    if (elect_one() && ok) {
 #pragma unroll
                         for (int t = first; t < kTiles; t += kIssuers)
                             if (t < w.n_mt) qk(t, 0, 0, item_slab(w, 0));
                     }
                     __syncwarp();
                 }
-                // A wait that gives up does not end the key loop (its result would make the loop's control flow, and with it
-                // the operands, non-uniform): the remaining waits of the item return at once and the item loop ends.
                 while (have) {
                     // key tiles with a successor in the same item
                     for (int j = 0; j < w.n_kv - 1; ++j) {
+                        if ((j & 31) == 31 && !__all_sync(0xffffffffu, ok)) {
+                            ok = false;
+                            break;
+                        }
                         const uint32_t st2 = (st + 1) % kStages;
                         if (st2 == 0) kv_phase ^= 1u;
-                        mbar_wait(&sh.kv_full[st2], kv_phase, sh, status, kErrKvFull);
+                        wait(sh.kv_full[st2], kv_phase, kErrKvFull);
                         const bool slab2 = item_slab(w, j + 1);
 #pragma unroll
                         for (int t = first; t < kTiles; t += kIssuers) {
                             if (t < w.n_mt) {
                                 // O_t += P_t V, then the next scores of the tile over P_t: the tensor core executes them in order
-                                mbar_wait(&sh.p_full[t], (p_phase >> t) & 1, sh, status, kErrPFull);
+                                wait(sh.p_full[t], (p_phase >> t) & 1, kErrPFull);
                                 p_phase ^= 1u << t;
                                 __syncwarp();
                                 tc_fence_after();
-                                if (elect_one()) {
+                                if (elect_one() && ok) {
                                     pv(t, st, j > 0 ? 1u : 0u);
                                     qk(t, st2, qb, slab2);
                                 }
                                 __syncwarp();
                             }
                         }
-                        if (elect_one()) tc_commit_1(&sh.kv_empty[st]);
+                        if (elect_one() && ok) tc_commit_1(&sh.kv_empty[st]);
                         __syncwarp();
                         st = st2;
                     }
@@ -787,8 +824,8 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                     bool slab2 = false;
                     if (st2 == 0) kv_phase ^= 1u;
                     if (have2) {
-                        mbar_wait(&sh.kv_full[st2], kv_phase, sh, status, kErrKvFull);
-                        mbar_wait(&sh.q_full[qb ^ 1], (q_phase >> (qb ^ 1)) & 1, sh, status, kErrQFull);
+                        wait(sh.kv_full[st2], kv_phase, kErrKvFull);
+                        wait(sh.q_full[qb ^ 1], (q_phase >> (qb ^ 1)) & 1, kErrQFull);
                         q_phase ^= 1u << (qb ^ 1);
                         slab2 = item_slab(nx, 0);
                     } else {
@@ -798,12 +835,12 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
 #pragma unroll
                     for (int t = first; t < kTiles; t += kIssuers) {
                         if (t < w.n_mt) {
-                            mbar_wait(&sh.p_full[t], (p_phase >> t) & 1, sh, status, kErrPFull);
+                            wait(sh.p_full[t], (p_phase >> t) & 1, kErrPFull);
                             p_phase ^= 1u << t;
                         }
                         __syncwarp();
                         tc_fence_after();
-                        if (elect_one()) {
+                        if (elect_one() && ok) {
                             if (t < w.n_mt) {
                                 pv(t, st, multi);
                                 tc_commit_1(&sh.o_done[t]);
@@ -812,20 +849,22 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                         }
                         __syncwarp();
                     }
-                    if (elect_one()) {
+                    if (elect_one() && ok) {
                         tc_commit_1(&sh.kv_empty[st]);
                         tc_commit_1(&sh.q_empty[qb]);
                     }
                     __syncwarp();
                     st = st2;
                     qb ^= 1u;
-                    ++items;
                     item = item2;
                     w = nx;
-                    have = have2 && __all_sync(0xffffffffu, sh.abort_flag == 0);
+                    have = have2 && __all_sync(0xffffffffu, ok && sh.abort_flag == 0);
                 }
-                // the last commits have arrived before the CTA may end
-                if (items > 0) mbar_wait(&sh.q_empty[qb ^ 1], ((items - 1) >> 1) & 1, sh, status, kErrQFull);
+                // all tensor-core work and all its commits have arrived before the CTA may end
+                __syncwarp();
+                if (elect_one()) tc_commit_1(&sh.drained);
+                __syncwarp();
+                mbar_drain(&sh.drained, 0, status, kErrODone);
                 __syncwarp();
             };
             if (warp == kIssuerWarp0) run(std::integral_constant<int, 0>{});
@@ -961,10 +1000,6 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     // ===== common exit ==========================================================================================
     tc_fence_before();
     __syncthreads();
-    if (sh.abort_flag != 0) {
-        // give loads that may still be in flight time to land before the shared memory is released
-        for (int i = 0; i < 64; ++i) __nanosleep(1000);
-    }
     if (warp == kIssuerWarp0) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(sh.tmem_base), "r"(kTmemCols) : "memory");
@@ -1077,7 +1112,7 @@ bool attn_sm100_supported(const AttnArgs &a) {
 // and a failed attempt is retried by the next launch.
 template <typename Kernel> static int ensure_smem_optin(Kernel kernel, int slot, size_t smem) {
     static std::mutex mu;
-    static bool done[64][4];
+    static bool done[64][5];
     int dev = 0;
     COME_CUDA(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64) {
@@ -1142,21 +1177,23 @@ int attn_sm100_launch(const AttnArgs &a, cudaStream_t stream) {
     const unsigned grid = (unsigned)(items < sms ? items : sms);  // persistent: one CTA per SM walks the items
     const float scale_log2 = a.scale * kLog2e;
     const float inv_scale = 1.0f / a.scale;
-#define COME_ATTN_LAUNCH(BF16, PREFIX, SLOT)                                                                                   \
+#define COME_ATTN_LAUNCH(BF16, PREFIX, SELFTEST, SLOT)                                                                         \
     do {                                                                                                                       \
-        if ((rc = ensure_smem_optin(attn_fwd_sm100_kernel<BF16, PREFIX>, SLOT, smem)) != COME_OK) return rc;                    \
-        attn_fwd_sm100_kernel<BF16, PREFIX><<<grid, kThreads, smem, stream>>>(mq, mk, mv, a.bias, a.cu, scale_log2, inv_scale, a.out, \
+        if ((rc = ensure_smem_optin(attn_fwd_sm100_kernel<BF16, PREFIX, SELFTEST>, SLOT, smem)) != COME_OK) return rc;          \
+        attn_fwd_sm100_kernel<BF16, PREFIX, SELFTEST><<<grid, kThreads, smem, stream>>>(mq, mk, mv, a.bias, a.cu, scale_log2, inv_scale, a.out, \
                                                                               a.o_rs, a.lse, (int)a.q_begin, (int)a.q_end, tiles, (int)span, \
                                                                               a.nseg, a.H, a.max_seqlen_dev, status, (int)a.total,   \
                                                                               a.q_free ? 1 : 0, split_tail, k_parts, (long long)a.part_o, \
-                                                                              (long long)a.part_l);                                  \
+                                                                              (long long)a.part_l, a.stall_tile);                    \
     } while (0)
-    if (a.dtype == COME_BF16) {
-        if (with_table) COME_ATTN_LAUNCH(true, true, 0);
-        else COME_ATTN_LAUNCH(true, false, 1);
+    if (a.stall_tile >= 0) {
+        COME_ATTN_LAUNCH(true, false, true, 4);
+    } else if (a.dtype == COME_BF16) {
+        if (with_table) COME_ATTN_LAUNCH(true, true, false, 0);
+        else COME_ATTN_LAUNCH(true, false, false, 1);
     } else {
-        if (with_table) COME_ATTN_LAUNCH(false, true, 2);
-        else COME_ATTN_LAUNCH(false, false, 3);
+        if (with_table) COME_ATTN_LAUNCH(false, true, false, 2);
+        else COME_ATTN_LAUNCH(false, false, false, 3);
     }
 #undef COME_ATTN_LAUNCH
     return check_launch("come_attn_varlen_fwd (tcgen05 kernel)");
@@ -1170,4 +1207,33 @@ extern "C" int come_selftest_bounded_wait(int64_t ticks, int64_t *waited_dev, vo
     if (!status) return COME_ERR_CUDA;
     come::selftest_wait_kernel<<<1, 32, 0, (cudaStream_t)stream>>>((long long)ticks, status, (long long *)waited_dev);
     return come::check_launch("come_selftest_bounded_wait");
+}
+
+extern "C" int come_selftest_attn_stall(const void *qkv_dev, int64_t total, int num_heads, const int32_t *cu_seqlens_dev, float softmax_scale,
+                                        int key_tiles, void *out_dev, float *lse_dev, void *stream) {
+    COME_REQUIRE(qkv_dev && cu_seqlens_dev && out_dev, "come_selftest_attn_stall: qkv, cu_seqlens and out must be given");
+    COME_REQUIRE(total > 0 && total < (1ll << 20) && num_heads > 0 && num_heads <= 64, "come_selftest_attn_stall: a small launch only (tokens below 2^20, at most 64 heads)");
+    COME_REQUIRE(key_tiles >= 0, "come_selftest_attn_stall: key_tiles must not be negative");
+    come::AttnArgs a = {};
+    const int64_t part = (int64_t)num_heads * come::kHeadDim;  // elements of q, of k and of v in a packed row
+    const uint16_t *qkv = static_cast<const uint16_t *>(qkv_dev);
+    a.q = qkv;
+    a.k = qkv + part;
+    a.v = qkv + 2 * part;
+    a.cu = cu_seqlens_dev;
+    a.out = out_dev;
+    a.lse = lse_dev;
+    a.dtype = COME_BF16;
+    a.total = a.q_end = total;
+    a.H = num_heads;
+    a.D = come::kHeadDim;
+    a.q_rs = a.k_rs = a.v_rs = 3 * part;
+    a.o_rs = part;
+    a.nseg = 1;
+    a.max_seqlen = (int)total;
+    a.scale = softmax_scale;
+    a.k_parts = 1;
+    a.stall_tile = key_tiles;
+    COME_REQUIRE(come::attn_sm100_supported(a), "come_selftest_attn_stall: needs 16-byte aligned tensors and a positive scale");
+    return come::attn_sm100_launch(a, (cudaStream_t)stream);
 }

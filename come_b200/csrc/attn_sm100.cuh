@@ -22,6 +22,8 @@ struct AttnArgs {
     // with few items per SM).  Share p writes out + p * part_o (elements) and lse + p * part_l (floats).
     int k_parts = 1;
     int64_t part_o = 0, part_l = 0;
+    // Self-test launches (bfloat16, one segment): every CTA's producer stops in front of its key tile `stall_tile`.
+    int stall_tile = -1;
 };
 
 // True when the tensor-core kernel can take the problem (head_dim 64, TMA-compatible addresses and strides).

@@ -374,6 +374,16 @@ int come_device_status(uint32_t *value, int clear);
 int come_selftest_bounded_wait(int64_t ticks, int64_t *waited_dev, void *stream);
 
 /*
+ * Self-test of the attention kernel's way out of a wait that ran out: bfloat16 self-attention of one segment on packed qkv
+ * [total, 3, num_heads, 64] (out [total, num_heads, 64], lse [num_heads, total] or NULL, cu_seqlens [2] = {0, total}), where
+ * every CTA loads its first `key_tiles` key tiles only.  The waits for the next one give up after 2^29 clock ticks (a third
+ * of a second), raise a bit of 0-9 of the device status word, and the kernel returns normally.  Rows of out / lse are then
+ * either what come_attn_varlen_fwd computes or untouched.  Clear the word afterwards.  No counterpart in the reference.
+ */
+int come_selftest_attn_stall(const void *qkv_dev, int64_t total, int num_heads, const int32_t *cu_seqlens_dev,
+                             float softmax_scale, int key_tiles, void *out_dev, float *lse_dev, void *stream);
+
+/*
  * Exchange of row blocks between the GPUs of one node through peer-mapped memory (one process per GPU): the transport of
  * the key / value all-gather of a global attention layer whose frames are sharded over the GPUs.  The reference has no
  * multi-GPU inference path; these entry points have no counterpart there.

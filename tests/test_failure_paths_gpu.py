@@ -3,6 +3,8 @@
 * the bounded wait of the attention kernel, exercised by the library's self-test (a barrier nothing arrives at, a
   limit of a fraction of a millisecond): the wait gives up, the status word is raised and reported, attention launches
   issued while it is raised return at once without touching their outputs, and clearing the word restores service;
+* the attention kernel's way out of a wait that ran out (key tiles that its producer never loads): the kernel returns, its
+  status is reported, every row of the result is right or untouched, and the next launch works;
 * every merge mask of up to 8 groups, for group sizes 1, 2, 3 and 9, bit-exact against the oracle;
 * outputs of merge, unmerge and attention placed between canary rows that must survive the launch.
 """
@@ -59,6 +61,42 @@ def test_bounded_wait_gives_up_and_is_reported():
         _lib.device_status(clear=True)
     with pytest.raises(RuntimeError, match="ticks"):
         _lib.check(lib.come_selftest_bounded_wait(1 << 40, None, None))
+
+
+@pytest.mark.parametrize("key_tiles", [0, 1, 5, 15, 16, 17, 31, 32])
+def test_attention_stall_leaves_rows_right_or_untouched(key_tiles):
+    """1000 keys are 16 key tiles, 2 heads x 8 query tiles on 2 CTAs: two items of four query tiles per CTA.  The waits run out
+    in front of the first tile (nothing in flight), inside the first item, at its end and in the second item; with all 32
+    key tiles of a CTA nothing runs out."""
+    from come_b200 import _lib, flash_attn_fwd_cuda as fa
+    from come_b200._torch_util import ptr, stream_ptr
+    P, H, D = 1000, 2, 64
+    rng = np.random.default_rng(3)
+    qkv = to_dev(rng.standard_normal((P, 3, H, D), dtype=np.float32), "bf16")
+    cu = torch.tensor([0, P], dtype=torch.int32, device="cuda")
+    assert _lib.device_status(clear=True) == 0
+    fa.set_backend(fa.BACKEND_TCGEN05)
+    try:
+        with fa.cta_limit(2):
+            want, want_lse = fa.varlen_fwd_rows(qkv[:, 0], qkv[:, 1], qkv[:, 2], cu, P, None, D ** -0.5, 0)
+            out = torch.full_like(want, 7.0)
+            lse = torch.full_like(want_lse, 7.0)
+            _lib.check(_lib.lib().come_selftest_attn_stall(ptr(qkv), P, H, ptr(cu), D ** -0.5, key_tiles, ptr(out), ptr(lse),
+                                                           stream_ptr(qkv.device)))
+            status = _lib.device_status(clear=True)
+            assert status >> 10 == 0 and (status != 0) == (key_tiles < 32), hex(status)
+            right = (out == want).all(dim=2).T & (lse == want_lse)     # [H, P]
+            untouched = (out == 7.0).all(dim=2).T & (lse == 7.0)
+            assert bool((right | untouched).all())
+            assert bool(untouched.any()) == (key_tiles < 32)  # the items that miss keys
+            if key_tiles != 16:
+                assert bool(right.any()) == (key_tiles > 16)  # the first items
+            again, again_lse = fa.varlen_fwd_rows(qkv[:, 0], qkv[:, 1], qkv[:, 2], cu, P, None, D ** -0.5, 0)
+        assert torch.equal(again, want) and torch.equal(again_lse, want_lse)
+        assert _lib.device_status(clear=True) == 0
+    finally:
+        fa.set_backend(fa.BACKEND_AUTO)
+        _lib.device_status(clear=True)
 
 
 @pytest.mark.parametrize("G", [1, 2, 3, 9])
