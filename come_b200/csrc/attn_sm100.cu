@@ -327,6 +327,8 @@ enum : uint32_t {
     kErrSFull = 1u << 5, kErrPFull = 1u << 7, kErrODone = 1u << 8, kErrTmem = 1u << 9,
     kErrSelfTest = 1u << 15,  // raised by the wait self-test on purpose
 };
+static_assert(((kErrQFull | kErrKvFull | kErrKvEmpty | kErrSFull | kErrPFull | kErrODone | kErrTmem) & ~kStatusAttention) == 0,
+              "come_device_status names these bits");
 
 // One work item = up to `tiles` 128-row query tiles [q_row0, q_row0 + tiles * 128) of one (segment, head).
 struct WorkItem {

@@ -50,6 +50,8 @@ int sm_count();
 // ---- device status word -----------------------------------------------------------------------------------
 // Address of the library's device status word on the current device (NULL and an error message on failure).
 unsigned int *status_word_dev();
+// Its bits that belong to the attention kernel (come_device_status names them as such).
+constexpr unsigned int kStatusAttention = 0x3ffu;
 
 // ---- element conversion -------------------------------------------------------------------------------------
 template <typename T> struct Elem;

@@ -357,8 +357,9 @@ int come_packed_positions(const uint8_t *mask_dev, const int64_t *rev_id_dev, in
  * Device status word: kernels that wait on hardware barriers give up after a bounded number of polls and
  * record a non-zero code here instead of hanging.  Reads it back (synchronises the device) and optionally
  * clears it.  Returns COME_OK with *value == 0 when no kernel reported a problem, COME_ERR_DEVICE with the word in
- * *value (and a message naming its bits) otherwise.  Bits 0-8: a wait of the attention kernel ran out (while the word is
- * raised, attention launches return at once without touching their outputs); bit 15: the wait self-test below; bit 16: a
+ * *value (and a message naming its bits) otherwise.  Bits 0-9: the attention kernel gave up, because a wait ran out (bits
+ * 0-8) or its tensor memory was not at column 0 (bit 9); while the word is raised, attention launches return at once without
+ * touching their outputs.  Bit 15: the wait self-test below; bit 16: a
  * position outside the rotary table was clamped by come_qkv_prepare; bit 17: a wait of the bulk-copy merge kernel ran out;
  * bit 18: come_peer_wait gave up.
  */
