@@ -20,7 +20,7 @@ EXPORTS = (
     "come_merge_plan_workspace_bytes", "come_merge_plan", "come_merge_plan_static", "come_merge", "come_merge_layernorm", "come_unmerge",
     "come_unmerge_strided", "come_unmerge_residual", "come_residual_layernorm", "come_suffix_add", "come_suffix_split",
     "come_attn_varlen_fwd", "come_attn_varlen_fwd_rows", "come_attn_cross_fwd", "come_attn_cross_fwd_parts", "come_attn_combine", "come_attn_combine_parts", "come_attn_set_cta_limit", "come_qkv_prepare", "come_packed_positions",
-    "come_device_status", "come_selftest_bounded_wait", "come_selftest_attn_stall",
+    "come_device_status", "come_selftest_bounded_wait", "come_selftest_attn_stall", "come_attn_work_list",
     "come_peer_alloc", "come_peer_open", "come_peer_close", "come_peer_free", "come_peer_copy", "come_peer_signal", "come_peer_wait",
 )
 COME_PEER_HANDLE_BYTES = 64
@@ -84,6 +84,7 @@ def lib() -> C.CDLL:
     l.come_packed_positions.argtypes = [vp, vp, i64, C.POINTER(Layout), vp, vp]
     l.come_device_status.argtypes = [C.POINTER(C.c_uint32), i32]
     l.come_selftest_bounded_wait.argtypes = [i64, vp, vp]
+    l.come_attn_work_list.argtypes = [vp, i32, i32, i64, i64, i32, vp, i32, vp, i64, vp]
     l.come_selftest_attn_stall.argtypes = [vp, i64, i32, vp, f32, i32, vp, vp, vp]
     l.come_peer_alloc.argtypes = [i64, C.POINTER(vp), vp]
     l.come_peer_open.argtypes = [vp, C.POINTER(vp)]

@@ -56,8 +56,8 @@ constexpr int kIssuers = 2;       // warps that issue the tensor-core work, two 
 constexpr int kIssuerWarp0 = kProducerWarp + 1;
 constexpr int kThreads = 32 * (kProducerWarp + 4);  // 640: four softmax warpgroups + one with the producer, the issuers and an idle warp
 static_assert(kTiles % kIssuers == 0 && 1 + kIssuers <= 4, "one warpgroup holds the producer and the issuers");
-// Launches with this many segments enumerate only the query blocks that exist (a prefix table in shared memory)
-constexpr int kMinPrefixSegs = 16, kMaxPrefixSegs = 2048;
+// Launches with this many segments keep a prefix table of their query blocks in shared memory; with fewer, a sorted list
+constexpr int kMinPrefixSegs = 16, kMaxPrefixSegs = 2048, kMaxListSegs = kMinPrefixSegs - 1;
 constexpr int kQTileBytes = kBlockM * kHeadDim * 2;   // 16384
 constexpr int kKvTileBytes = kBlockN * kHeadDim * 2;  // 8192
 constexpr int kQSlabBytes = kBlockM * 16 * 2, kSlabBytes = kBlockN * 16 * 2;  // 16 columns of 16 bits
@@ -96,8 +96,14 @@ struct SharedStorage {
     uint64_t drained;         // all tensor-core work of the CTA complete (exit path)
     uint32_t tmem_base;
     volatile uint32_t abort_flag;
-    int scan_warp[kThreads / 32];
-    int height_sums[2 * kTiles];
+    // work list (see plan_work)
+    int4 seg_rows[kMaxListSegs];            // keys [x, y) and query rows [z, w) of a segment, by falling number of keys
+    int4 seg_items[kTiles][kMaxListSegs];   // [height - 1]: first item of the segment, items per head, their reciprocal
+    int4 plan[kTiles];                      // [height - 1]: items, first item of a split last round, its parts, their reciprocal
+    float plan_cost[kTiles];
+    uint32_t per_head_rcp;
+    int scan_warp[kThreads / 32], sum_items[kTiles][kThreads / 32];
+    float sum_cost[kTiles][kThreads / 32];
 };
 // Launches that use the prefix table get (kMaxPrefixSegs + 1) ints of dynamic shared memory behind SharedStorage:
 // table[s] = query blocks of the segments before s (this launch's rows).
@@ -340,10 +346,19 @@ struct WorkItem {
     int kpart;          // which share of the keys this item covers (launches that split the keys of their items), else 0
 };
 
-// 128-row query tiles of segment `seg` that hold rows of this launch.
-__device__ __forceinline__ int segment_tiles(int seg, const int *__restrict__ cu, int q_begin, int q_end) {
-    const int rows = min(cu[seg + 1], q_end) - max(cu[seg], q_begin);
-    return rows > 0 ? (rows + kBlockM - 1) / kBlockM : 0;
+__host__ __device__ constexpr int tiles_of(int rows) { return rows > 0 ? (rows + kBlockM - 1) / kBlockM : 0; }
+__host__ __device__ constexpr int key_tiles_of(int keys) { return keys > 0 ? (keys + kBlockN - 1) / kBlockN : 0; }
+
+// n / d and the remainder by the reciprocal floor((2^32 - 1) / d), for any 32-bit n: the estimate is at most one too small.
+__device__ __forceinline__ uint32_t reciprocal(int d) { return d > 0 ? 0xffffffffu / (uint32_t)d : 0u; }
+__device__ __forceinline__ int div_by(int n, int d, uint32_t rcp, int &rem) {
+    int q = (int)__umulhi((uint32_t)n, rcp);
+    rem = n - q * d;
+    if (rem >= d) {
+        ++q;
+        rem -= d;
+    }
+    return q;
 }
 
 // Query tiles per work item.  A key step of an item costs less than in proportion to its tiles (the tiles share the SM's
@@ -351,12 +366,11 @@ __device__ __forceinline__ int segment_tiles(int seg, const int *__restrict__ cu
 // best where there are many items; but the items are dealt to the CTAs in rounds, and with few of them the height that
 // fills its last round wins: 6456 tokens x 16 heads take 215 us with 3 (272 items, 2 rounds) and 260 with 4 (208 items, also
 // 2 rounds); 3228 tokens 59 and 68 us; 2 segments of ~450 tokens 12.0 us with 1 and 16.8 with 4; 4 x 807 tokens 24 us with
-// 4 and 37 with 3.  The choice is the height with the least (full rounds of items over the CTAs) x (mean cost of an item) + the last
-// round, whose items are split into lower ones where the CTAs suffice for that (tail_height): 24,576 tokens x 16 heads are
-// 768 items = 5 rounds + 28 items of four tiles, which run as 112 items of one (3.02 -> 2.87 ms); 80,672 tokens are 17
-// rounds + 12 items (30.6 -> 29.7 ms).  The
-// segments of a launch are known exactly on the device only, so every CTA makes the same choice from them (about 1 us of
-// the launch); the host makes it for one segment, and where every query tile gets a CTA of its own.
+// 4 and 37 with 3.  The choice is the height with the least sum, over the rounds, of the mean cost of an item of the segment the
+// round begins in (its step by its key tiles); the items of a partial last round are split into lower ones where the CTAs
+// suffice for that (tail_height): 24,576 tokens x 16 heads are 768 items = 5 rounds + 28 items of four tiles, which run as 112
+// items of one (3.02 -> 2.87 ms); 80,672 tokens are 17 rounds + 12 items (30.6 -> 29.7 ms).  The step costs were measured at
+// 6456 keys; what an item costs beyond its steps is not in them.
 __host__ __device__ __forceinline__ int step_cost(int n) { return n <= 0 ? 0 : n == 1 ? 70 : n == 2 ? 80 : n == 3 ? 96 : 115; }
 // Height of the items of the last, partial round of `rest` items of `height` tiles.
 __host__ __device__ __forceinline__ int tail_height(int height, int rest, int ctas) {
@@ -364,106 +378,294 @@ __host__ __device__ __forceinline__ int tail_height(int height, int rest, int ct
     if (height > 2 && rest * 2 <= ctas) return 2;
     return height;
 }
-struct HeightSums {
-    int items[kTiles], cost[kTiles];  // [height - 1], of one head
-    __host__ __device__ __forceinline__ void add(int n) {
+__host__ __device__ __forceinline__ int blocks_of(int n, int height) {  // items of n query tiles
+    return height == 1 ? n : height == 2 ? (n + 1) >> 1 : height == 4 ? (n + 3) >> 2 : (n + 2) / 3;
+}
+__host__ __device__ __forceinline__ int height_cost(int n, int height) {  // of these items
+    const int blocks = blocks_of(n, height), rest = n - (blocks - 1) * height;
+    return n <= 0 ? 0 : (blocks - 1) * step_cost(height) + step_cost(rest);
+}
+
+// Work list of a launch: the items [0, total) of `height` query tiles, of which those from `from` on are split into `parts`
+// lower ones, and how an item becomes rows of a segment and a head.  Planned on the host where it knows enough, else by every
+// CTA for itself.
+//  * One segment, launches in which every query tile gets a CTA of its own or no segment has a second one (height 1), and
+//    those with more segments than the prefix table holds: planned on the host.  `slots` blocks for every (segment, head); those beyond a
+//    segment's end are skipped as invalid.
+//  * 2 .. kMaxListSegs segments (the sorted list): the items are exactly those that exist, in the order (segment by falling
+//    number of keys, head, block).  Dealt round-robin the CTAs then get items of like length in every round and the short ones
+//    fill up at the end.  One slot per segment and maximal block in the order (head, segment, block) costs segments of unlike
+//    length up to 2.7 x: 12000 + 6000 + 3000 + 1500 + 750 + 375 tokens x 6 heads took 1349 us (the long segment's blocks
+//    of all heads fall on the same CTAs) and take 350; 20000 + 10 x 500 tokens x 16 heads 3817 and 1908.
+//  * kMinPrefixSegs .. kMaxPrefixSegs segments (the prefix table): the items that exist in the order (head, segment, block).
+// Warps 0 .. kTiles - 1 plan one height each while other warps initialise the barriers and allocate tensor memory; after the
+// barrier every thread picks the cheapest.  What a short launch feels is the code that runs once, at 4 to 5 clocks per
+// instruction: planned by every warp for itself, in each other's issue slots, the same took 3250 clocks.
+struct WorkPlan {
+    int height;  // 0: planned on the device
+    int total, from, parts, slots;
+    uint32_t parts_rcp, slots_rcp, nseg_rcp, ctas_rcp;
+};
+struct WorkArgs {
+    const int *cu;        // may be NULL for q_free: [0, kv_total]
+    int nseg, num_heads, q_begin, q_end, kv_total, max_rows, k_parts, ctas;
+    bool q_free;
+};
+
+// Cost of a plan of `height` whose rounds cost `cost`, of which the last, partial one has `rest` items of `mean` cost and
+// `keys` key tiles: its items are split into lower ones where the CTAs suffice.
+__host__ __device__ __forceinline__ float split_last_round(WorkPlan &pl, int height, int items, int rest, float cost, float mean, float keys, int ctas) {
+    pl.height = height;
+    pl.total = pl.from = items;
+    pl.parts = 1;
+    pl.parts_rcp = 0xffffffffu;
+    const int low = tail_height(height, rest, ctas);
+    if (rest > 0 && low != height) {
+        pl.parts = low == 2 ? 2 : height;
+        pl.parts_rcp = pl.parts == 2 ? 0x7fffffffu : pl.parts == 3 ? 0x55555555u : 0x3fffffffu;
+        pl.from = items - rest;
+        pl.total = pl.from + rest * pl.parts;
+        cost += (float)step_cost(low) * keys - mean;
+    }
+    return cost;
+}
+__device__ __forceinline__ void store_plan(SharedStorage &sh, const WorkPlan &pl, float cost) {
+    sh.plan[pl.height - 1] = make_int4(pl.total, pl.from, pl.parts, (int)pl.parts_rcp);
+    sh.plan_cost[pl.height - 1] = cost;
+}
+
+// The sorted list for items of `height` tiles, by one warp: a lane per segment.
+__device__ __forceinline__ void plan_list(SharedStorage &sh, const WorkArgs &a, const WorkPlan &host, int height, int lane) {
+    int4 rows = make_int4(0, 0, 0, 0);
+    if (lane < a.nseg) {
+        rows.x = a.cu[lane];
+        rows.y = a.cu[lane + 1];
+        rows.z = max(rows.x, a.q_begin);
+        rows.w = min(rows.y, a.q_end);
+    }
+    const int keys = key_tiles_of(rows.y - rows.x), n = tiles_of(min(rows.w - rows.z, a.max_rows));
+    const int blocks = blocks_of(n, height);
+    int rank = 0, first = 0;
+#pragma unroll 1
+    for (int j = 0; j < a.nseg; ++j) {
+        const int other_keys = __shfl_sync(0xffffffffu, keys, j), other_blocks = __shfl_sync(0xffffffffu, blocks, j);
+        const bool before = other_keys > keys || (other_keys == keys && j < lane);
+        rank += before ? 1 : 0;
+        first += before ? other_blocks : 0;
+    }
+    first *= a.num_heads;
+    const int end = first + blocks * a.num_heads;
+    if (lane < a.nseg) {
+        if (height == kTiles) sh.seg_rows[rank] = rows;
+        sh.seg_items[height - 1][rank] = make_int4(first, blocks, (int)reciprocal(blocks), 0);
+    }
+    int rem;
+    const int rounds_before = div_by(first + a.ctas - 1, a.ctas, host.ctas_rcp, rem);  // rounds that begin in front of the segment
+    const int rounds = div_by(end + a.ctas - 1, a.ctas, host.ctas_rcp, rem) - rounds_before;
+    const float mean = blocks > 0 ? __fdividef((float)height_cost(n, height), (float)blocks) * (float)keys : 0.0f;
+    float cost = (float)rounds * mean;
 #pragma unroll
-        for (int h = 1; h <= kTiles; ++h) {
-            items[h - 1] += (n + h - 1) / h;
-            cost[h - 1] += (n / h) * step_cost(h) + step_cost(n % h);
+    for (int d = 8; d > 0; d >>= 1) cost += __shfl_xor_sync(0xffffffffu, cost, d);  // lanes 0 .. 15
+    const int items = (int)__reduce_max_sync(0xffffffffu, (unsigned)end);
+    int rest;
+    div_by(items, a.ctas, host.ctas_rcp, rest);
+    const unsigned owner = __ballot_sync(0xffffffffu, first <= items - rest && items - rest < end);
+    const int src = max(__ffs(owner) - 1, 0);
+    const float last = __shfl_sync(0xffffffffu, mean, src);
+    const int last_keys = __shfl_sync(0xffffffffu, keys, src);
+    if (lane == 0) {
+        WorkPlan pl;
+        cost = split_last_round(pl, height, items, rest, cost, last, (float)last_keys, a.ctas);
+        store_plan(sh, pl, cost);
+    }
+}
+
+__device__ __forceinline__ int cheapest_height(const SharedStorage &sh) {  // the greatest of equally cheap ones
+    int height = kTiles;
+    float least = sh.plan_cost[kTiles - 1];
+#pragma unroll
+    for (int h = kTiles - 1; h >= 1; --h) {
+        const float cost = sh.plan_cost[h - 1];
+        if (cost < least) {
+            least = cost;
+            height = h;
         }
     }
-    __device__ __forceinline__ void warp_sum() {
+    return height;
+}
+
+// The prefix table, by the whole CTA: a height from the sums over all segments, then a scan of the query blocks.  The sums
+// are formed in a fixed order, so that every CTA makes the same choice.  Returns the height.
+__device__ __forceinline__ int plan_prefix(SharedStorage &sh, const WorkArgs &a, const WorkPlan &host, int *prefix) {
+    constexpr int kPer = (kMaxPrefixSegs + kThreads) / kThreads;  // consecutive segments per thread
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int local[kPer], items[kTiles] = {};
+    float cost[kTiles] = {};
 #pragma unroll
-        for (int h = 0; h < kTiles; ++h) {
-            items[h] = __reduce_add_sync(0xffffffffu, items[h]);
-            cost[h] = __reduce_add_sync(0xffffffffu, cost[h]);
-        }
-    }
-    __host__ __device__ __forceinline__ int best(int num_heads, int ctas) const {
-        int height = kTiles;
-        float least = 3.0e38f;
+    for (int i = 0; i < kPer; ++i) {
+        const int sg = threadIdx.x * kPer + i;
+        local[i] = 0;
+        if (sg < a.nseg) {
+            const int s0 = a.cu[sg], s1 = a.cu[sg + 1];
+            local[i] = tiles_of(min(s1, a.q_end) - max(s0, a.q_begin));
+            const float keys = (float)key_tiles_of(s1 - s0);
 #pragma unroll
-        for (int h = kTiles; h >= 1; --h) {
-            const int n = items[h - 1] * num_heads, rest = n % ctas, low = tail_height(h, rest, ctas);
-            const float mean = (float)cost[h - 1] / (float)(items[h - 1] > 0 ? items[h - 1] : 1);
-            const float t = (float)(n / ctas) * mean + (rest == 0 ? 0.0f : low == h ? mean : (float)step_cost(low));
-            if (t < least) {
-                least = t;
-                height = h;
+            for (int h = 1; h <= kTiles; ++h) {
+                items[h - 1] += blocks_of(local[i], h);
+                cost[h - 1] += keys * (float)height_cost(local[i], h);
             }
         }
-        return height;
     }
-};
+#pragma unroll
+    for (int h = 0; h < kTiles; ++h) {
+        items[h] = (int)__reduce_add_sync(0xffffffffu, (unsigned)items[h]);
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) cost[h] += __shfl_xor_sync(0xffffffffu, cost[h], d);
+        if (lane == 0) {
+            sh.sum_items[h][warp] = items[h];
+            sh.sum_cost[h][warp] = cost[h];
+        }
+    }
+    __syncthreads();
+    if (warp < kTiles) {
+        const bool has = lane < kThreads / 32;
+        const int total = a.num_heads * (int)__reduce_add_sync(0xffffffffu, has ? (unsigned)sh.sum_items[warp][lane] : 0u);
+        float sum = has ? sh.sum_cost[warp][lane] : 0.0f;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+        if (lane == 0) {
+            const float mean = sum * (float)a.num_heads / (float)max(total, 1);
+            int rest;
+            int rounds = div_by(total, a.ctas, host.ctas_rcp, rest);
+            rounds += rest > 0 ? 1 : 0;
+            WorkPlan pl;
+            const float all = split_last_round(pl, warp + 1, total, rest, (float)rounds * mean, mean, mean / (float)step_cost(warp + 1), a.ctas);
+            store_plan(sh, pl, all);
+        }
+    }
+    __syncthreads();
+    const int height = cheapest_height(sh);
+    int sum = 0;
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+        local[i] = blocks_of(local[i], height);
+        sum += local[i];
+    }
+    int incl = sum;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += v;
+    }
+    if (lane == 31) sh.scan_warp[warp] = incl;
+    __syncthreads();
+    int before = incl - sum;
+    for (int wq = 0; wq < warp; ++wq) before += sh.scan_warp[wq];
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+        const int sg = threadIdx.x * kPer + i;
+        if (sg <= a.nseg) prefix[sg] = before;
+        if (sg == a.nseg) sh.per_head_rcp = reciprocal(before);
+        before += local[i];
+    }
+    return height;
+}
 
-// The items from `from` on (the last, partial round) are split into `parts` items of `tiles` query tiles.
-struct TailSplit {
-    int from, parts, tiles;
-};
+// Plans the launch; after the caller's next __syncthreads picked_height names the height.  Returns that of a table launch.
+template <bool kPrefix>
+__device__ __forceinline__ int plan_work(SharedStorage &sh, const WorkArgs &a, const WorkPlan &host, int *prefix) {
+    if constexpr (kPrefix) {
+        return plan_prefix(sh, a, host, prefix);
+    } else {
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        if (host.height == 0) {
+            if (warp < kTiles) plan_list(sh, a, host, warp + 1, lane);
+        } else if (threadIdx.x == 0) {
+            store_plan(sh, host, 0.0f);
+            if (a.nseg == 1) {
+                const int s0 = a.cu ? a.cu[0] : 0, s1 = a.cu ? a.cu[1] : a.kv_total;
+                sh.seg_rows[0] = make_int4(s0, s1, a.q_free ? a.q_begin : max(s0, a.q_begin), a.q_free ? a.q_end : min(s1, a.q_end));
+            }
+        }
+        return 0;
+    }
+}
+__device__ __forceinline__ int picked_height(const SharedStorage &sh, int planned, const WorkPlan &host) {
+    return planned != 0 ? planned : host.height != 0 ? host.height : cheapest_height(sh);
+}
 
-// Item -> (head, segment, query block).  With a prefix table (seg_prefix != nullptr) the items are exactly the query
-// blocks that exist, in (head, segment, block) order; without it every segment gets `nblk_x` slots and the surplus ones
-// are skipped as invalid.
+// Item -> (head, segment, query block), by a converged warp.
 // q_free: the launch has one segment whose keys all query rows [q_begin, q_end) attend to, whether or not those rows lie
 // inside the segment (attention of this GPU's rows to keys gathered from other GPUs); cu may then be NULL = [0, kv_total].
 template <bool kPrefix>
-__device__ __forceinline__ WorkItem decode_item(int item, int nblk_x, int nseg, const int *__restrict__ cu, int q_begin, int q_end,
-                                                const int *seg_prefix, int kv_total, bool q_free, int tiles, int k_parts,
-                                                const TailSplit &tail) {
+__device__ __forceinline__ WorkItem decode_item(int item, const SharedStorage &sh, const WorkArgs &a, const WorkPlan &host, const int *prefix,
+                                                int height) {
     WorkItem w;
-    int bx, seg;
+    int bx, q_lo;
+    int first_tile = 0, most_tiles = height;  // of the item's rows inside its block of `height` tiles
+    const int4 pl = sh.plan[height - 1];
+    if (item >= pl.y) {
+        const int i = div_by(item - pl.y, pl.z, (uint32_t)pl.w, first_tile);
+        item = pl.y + i;
+        most_tiles = pl.z == height ? 1 : 2;
+        first_tile *= most_tiles;
+    }
     // Launches with k_parts > 1 (q_free only): consecutive items are the shares of the key tiles of one (head, block); every
     // share writes its own output and log-sum-exp, merged afterwards.  The host picks k_parts so that no share is empty.
     w.kpart = 0;
-    int sub = 0;  // position inside a split item
-    if (item >= tail.from) {
-        const int i = item - tail.from;
-        sub = i % tail.parts;
-        item = tail.from + i / tail.parts;
+    if (a.k_parts > 1) {
+        w.kpart = item % a.k_parts;
+        item /= a.k_parts;
     }
-    const bool split = tail.parts > 1 && item >= tail.from;
-    if (k_parts > 1) {
-        w.kpart = item % k_parts;
-        item /= k_parts;
-    }
-    if constexpr (kPrefix) {
-        const int per_head = seg_prefix[nseg];
-        w.head = item / per_head;
-        const int r = item - w.head * per_head;
-        int lo = 0, hi = nseg;  // last segment whose prefix is <= r
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (seg_prefix[mid] <= r) lo = mid;
-            else hi = mid;
-        }
-        seg = lo;
-        bx = r - seg_prefix[seg];
-    } else {
-        bx = item % nblk_x;
-        const int rest = item / nblk_x;
-        seg = rest % nseg;
-        w.head = rest / nseg;
-    }
-    w.s0 = cu ? cu[seg] : 0;
-    w.s1 = cu ? cu[seg + 1] : kv_total;
-    const int seg_len = w.s1 - w.s0;
     // Query rows of this launch: global rows [q_begin, q_end) (the whole packed sequence for plain self-attention; a
     // slice when the query rows are sharded).  q / out / lse are indexed by (global row - q_begin); k / v by global row.
-    const int q_lo = q_free ? q_begin : max(w.s0, q_begin);
-    w.q_hi = q_free ? q_end : min(w.s1, q_end);
-    w.q_row0 = q_lo + bx * (tiles * kBlockM);
-    int rows = min(w.q_hi - w.q_row0, tiles * kBlockM);  // of the item
-    if (split) {
-        w.q_row0 += sub * (tail.tiles * kBlockM);
-        rows = min(rows - sub * (tail.tiles * kBlockM), tail.tiles * kBlockM);
+    if constexpr (kPrefix) {
+        int r;
+        w.head = div_by(item, prefix[a.nseg], sh.per_head_rcp, r);
+        int lo = 0, hi = a.nseg;  // last segment whose prefix is <= r
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (prefix[mid] <= r) lo = mid;
+            else hi = mid;
+        }
+        bx = r - prefix[lo];
+        w.s0 = a.cu[lo];
+        w.s1 = a.cu[lo + 1];
+        q_lo = max(w.s0, a.q_begin);
+        w.q_hi = min(w.s1, a.q_end);
+    } else if (host.height == 0 || a.nseg == 1) {
+        int rank = 0;
+        if (host.height == 0) {  // the last segment whose first item is not behind this one
+            const int lane = threadIdx.x & 31;
+            const int4 *list = sh.seg_items[height - 1];
+            rank = __popc(__ballot_sync(0xffffffffu, lane < a.nseg && list[min(lane, kMaxListSegs - 1)].x <= item)) - 1;
+            const int4 it = list[rank];
+            w.head = div_by(item - it.x, it.y, (uint32_t)it.z, bx);
+        } else {
+            w.head = div_by(item, host.slots, host.slots_rcp, bx);
+        }
+        const int4 rows = sh.seg_rows[rank];
+        w.s0 = rows.x;
+        w.s1 = rows.y;
+        q_lo = rows.z;
+        w.q_hi = rows.w;
+    } else {
+        int seg;
+        w.head = div_by(div_by(item, host.slots, host.slots_rcp, bx), a.nseg, host.nseg_rcp, seg);
+        w.s0 = a.cu[seg];
+        w.s1 = a.cu[seg + 1];
+        q_lo = max(w.s0, a.q_begin);
+        w.q_hi = min(w.s1, a.q_end);
     }
+    const int seg_len = w.s1 - w.s0;
+    w.q_row0 = q_lo + (bx * height + first_tile) * kBlockM;
+    const int rows = min(w.q_hi - w.q_row0, min(height - first_tile, most_tiles) * kBlockM);  // of the item
     w.valid = rows > 0;
     w.n_mt = (rows + kBlockM - 1) / kBlockM;  // query tiles with at least one valid row
     w.n_kv = (seg_len + kBlockN - 1) / kBlockN;
     w.ragged_tail = (seg_len % kBlockN) != 0;
-    if (k_parts > 1) {
-        const int per_part = (w.n_kv + k_parts - 1) / k_parts;
+    if (a.k_parts > 1) {
+        const int per_part = (w.n_kv + a.k_parts - 1) / a.k_parts;
         const int t0 = w.kpart * per_part, t1 = min(w.n_kv, t0 + per_part);
         if (t0 >= t1) {
             w.valid = false;
@@ -489,9 +691,9 @@ __global__ void __launch_bounds__(kThreads, 1)
 attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                       const __grid_constant__ CUtensorMap map_v, const void *__restrict__ bias_ptr,
                       const int *__restrict__ cu, float scale_log2, float inv_scale, void *__restrict__ out_ptr, int64_t o_rs,
-                      float *__restrict__ lse, int q_begin, int q_end, int tiles, int max_rows, int nseg, int num_heads,
-                      const int *__restrict__ max_len_dev, unsigned int *__restrict__ status, int kv_total, int q_free_flag, int split_tail,
-                      int k_parts, long long part_o, long long part_l, int stall_tile) {
+                      float *__restrict__ lse, int q_begin, int q_end, int max_rows, int nseg, int num_heads,
+                      const int *__restrict__ max_len_dev, unsigned int *__restrict__ status, int kv_total, int q_free_flag,
+                      int k_parts, long long part_o, long long part_l, const WorkPlan host_plan, int stall_tile) {
     using T = typename std::conditional<kBF16, __nv_bfloat16, __half>::type;
     // the declared alignment makes the base, and with it every barrier address and matrix descriptor, a link-time constant
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -499,101 +701,17 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
 
     // `max_rows` is the host's upper bound of the query rows of a segment.  A caller that cannot read the true length back
     // (a captured graph serving every merge mask) passes a loose bound plus the true one in device memory.
-    if (max_len_dev != nullptr) max_rows = min(max_rows, max(*max_len_dev, 0));
-    int nblk_x = 0;  // slots per segment of a launch without the prefix table
-    // Work list.  Launches with many segments (kMinPrefixSegs .. kMaxPrefixSegs): every CTA scans the segments' query-block
-    // counts into shared memory and the items are exactly the blocks that exist.  With ragged segments a list with one
-    // slot per (segment, maximal block index) unbalances the round-robin: the empty slots all carry the same block index,
-    // and 148 CTAs is a multiple of 4 blocks per segment (0.81 balance on 64 ragged segments, 0.95 without the empty
-    // slots).  Launches with few segments keep the slot list: the scan would cost them ~1.5 us for nothing.
-    constexpr bool use_prefix = kPrefix;  // the host instantiates and sizes the shared memory by the segment count
-    int *prefix_table = reinterpret_cast<int *>(reinterpret_cast<uint8_t *>(&sh) + sizeof(SharedStorage));
-    if constexpr (kPrefix) {
-        constexpr int kPer = (kMaxPrefixSegs + kThreads) / kThreads;  // consecutive segments per thread
-        int local[kPer], sum = 0;
-        HeightSums hs = {};
-#pragma unroll
-        for (int i = 0; i < kPer; ++i) {
-            const int sg = threadIdx.x * kPer + i;
-            local[i] = sg < nseg ? segment_tiles(sg, cu, q_begin, q_end) : 0;
-            hs.add(local[i]);
-        }
-        if (tiles == 0) {
-            if (threadIdx.x < 2 * kTiles) sh.height_sums[threadIdx.x] = 0;
-            __syncthreads();
-            hs.warp_sum();
-            if ((threadIdx.x & 31) == 0) {
-#pragma unroll
-                for (int h = 0; h < kTiles; ++h) {
-                    atomicAdd(&sh.height_sums[h], hs.items[h]);
-                    atomicAdd(&sh.height_sums[kTiles + h], hs.cost[h]);
-                }
-            }
-            __syncthreads();
-#pragma unroll
-            for (int h = 0; h < kTiles; ++h) {
-                hs.items[h] = sh.height_sums[h];
-                hs.cost[h] = sh.height_sums[kTiles + h];
-            }
-            tiles = hs.best(num_heads, gridDim.x);
-        }
-#pragma unroll
-        for (int i = 0; i < kPer; ++i) {
-            local[i] = (local[i] + tiles - 1) / tiles;
-            sum += local[i];
-        }
-        int incl = sum;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, incl, d);
-            if ((threadIdx.x & 31) >= d) incl += v;
-        }
-        if ((threadIdx.x & 31) == 31) sh.scan_warp[threadIdx.x >> 5] = incl;
-        __syncthreads();
-        int before = incl - sum;
-        for (int wq = 0; wq < (int)(threadIdx.x >> 5); ++wq) before += sh.scan_warp[wq];
-#pragma unroll
-        for (int i = 0; i < kPer; ++i) {
-            const int sg = threadIdx.x * kPer + i;
-            if (sg <= nseg) prefix_table[sg] = before;
-            before += local[i];
-        }
-        __syncthreads();
-    }
-    if constexpr (!kPrefix) {
-        const int lane_seg = threadIdx.x & 31;
-        if (tiles == 0) {  // fewer than kMinPrefixSegs segments: a lane each, every warp on its own
-            int n = lane_seg < nseg ? segment_tiles(lane_seg, cu, q_begin, q_end) : 0;
-            n = min(n, (max_rows + kBlockM - 1) / kBlockM);
-            HeightSums hs = {};
-            hs.add(n);
-            hs.warp_sum();
-            tiles = hs.best(num_heads, gridDim.x);
-            nblk_x = (__reduce_max_sync(0xffffffffu, n) + tiles - 1) / tiles;
-        } else {
-            nblk_x = (max_rows + tiles * kBlockM - 1) / (tiles * kBlockM);
-        }
-    }
-    const int *seg_prefix = use_prefix ? prefix_table : nullptr;
-    int total_items = (use_prefix ? prefix_table[nseg] * num_heads : nblk_x * nseg * num_heads) * k_parts;
-    TailSplit tail{total_items, 1, tiles};
-    if (split_tail) {
-        const int rest = total_items % (int)gridDim.x;
-        tail.tiles = tail_height(tiles, rest, gridDim.x);
-        if (tail.tiles != tiles) {
-            tail.parts = (tiles + tail.tiles - 1) / tail.tiles;
-            tail.from = total_items - rest;
-            total_items = tail.from + rest * tail.parts;
-        }
-    }
+    WorkArgs work{cu, nseg, num_heads, q_begin, q_end, kv_total, max_rows, k_parts, (int)gridDim.x, q_free_flag != 0};
+    if (max_len_dev != nullptr) work.max_rows = min(max_rows, max(*max_len_dev, 0));
+    int *prefix = reinterpret_cast<int *>(reinterpret_cast<uint8_t *>(&sh) + sizeof(SharedStorage));  // launches with the table
+    const int planned = plan_work<kPrefix>(sh, work, host_plan, prefix);
     const bool has_bias = bias_ptr != nullptr;
-    const bool q_free = q_free_flag != 0;
     // a key tile needs the bias step when there is a bias, or when it is the partial last tile (masking)
     auto uses_slab = [&](const WorkItem &w, int j) { return has_bias || (w.ragged_tail && j == w.n_kv - 1); };
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == 32 * kProducerWarp) {
         // an earlier CTA that gave up leaves the status word raised: later CTAs then skip their work
         sh.abort_flag = (*(volatile unsigned int *)status != 0) ? 1u : 0u;
         for (int i = 0; i < 2; ++i) {
@@ -620,6 +738,8 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    const int height = picked_height(sh, planned, host_plan);
+    const int total_items = sh.plan[height - 1].x;
     // All of the SM's tensor memory is allocated, so its base is column 0: the tensor-memory addresses are constants.
     constexpr uint32_t tmem = 0;
     // Register budget: the producer / issuer warpgroup needs few registers and hands its share to the softmax warpgroups
@@ -649,7 +769,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
             int it = 0;      // ring position = key tiles loaded so far
             int q_uses = 0;  // items whose Q was loaded so far (buffer and phase of q_full / q_empty)
             for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x) {
-                const WorkItem w = decode_item<kPrefix>(item, nblk_x, nseg, cu, q_begin, q_end, seg_prefix, kv_total, q_free, tiles, k_parts, tail);
+                const WorkItem w = decode_item<kPrefix>(item, sh, work, host_plan, prefix, height);
                 if (!w.valid) continue;
                 if (lane == 0) {
                     // Item n uses Q buffer n & 1, free once the last tensor-core work of item n - 2 has completed: the next
@@ -753,7 +873,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                 };
                 auto next_valid = [&](int &item, Item &x) -> bool {
                     for (; item < total_items; item += gridDim.x) {
-                        const WorkItem w = decode_item<kPrefix>(item, nblk_x, nseg, cu, q_begin, q_end, seg_prefix, kv_total, q_free, tiles, k_parts, tail);
+                        const WorkItem w = decode_item<kPrefix>(item, sh, work, host_plan, prefix, height);
                         if (w.valid) {
                             x = Item{w.n_mt, w.n_kv, w.ragged_tail};
                             return true;
@@ -883,7 +1003,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         bool ok = true;
         uint32_t s_phase = 0, o_phase = 0;
         for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x) {
-            const WorkItem w = decode_item<kPrefix>(item, nblk_x, nseg, cu, q_begin, q_end, seg_prefix, kv_total, q_free, tiles, k_parts, tail);
+            const WorkItem w = decode_item<kPrefix>(item, sh, work, host_plan, prefix, height);
             if (!w.valid || t >= w.n_mt) continue;
             const int n_kv = w.n_kv;
             float m_ref = -INFINITY, l = 0.0f;  // reference max (log2 units, scale applied) and running sum
@@ -1025,6 +1145,45 @@ __global__ void selftest_wait_kernel(long long ticks, unsigned int *__restrict__
     if (threadIdx.x == 0 && waited_out) *waited_out = ok ? -1 : clock64() - t0;
 }
 
+// The work list of a launch on `ctas` CTAs as the attention kernel walks it, for tests: out[0 .. 4) = items, query tiles per
+// item, first split item, parts of a split one; then per item head, first and last + 1 key, first query row, end of the query
+// rows, query tiles (0: skipped), key tiles
+template <bool kPrefix>
+__global__ void __launch_bounds__(kThreads, 1)
+work_list_kernel(const int *__restrict__ cu, int q_begin, int q_end, int max_rows, int nseg, int num_heads, const int *__restrict__ max_len_dev, int ctas,
+                 const WorkPlan host_plan, int *__restrict__ out, int capacity) {
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    SharedStorage &sh = *reinterpret_cast<SharedStorage *>(smem_raw);
+    WorkArgs work{cu, nseg, num_heads, q_begin, q_end, 0, max_rows, 1, ctas, false};
+    if (max_len_dev != nullptr) work.max_rows = min(max_rows, max(*max_len_dev, 0));
+    int *prefix = reinterpret_cast<int *>(reinterpret_cast<uint8_t *>(&sh) + sizeof(SharedStorage));
+    const int planned = plan_work<kPrefix>(sh, work, host_plan, prefix);
+    __syncthreads();
+    const int height = picked_height(sh, planned, host_plan);
+    const int4 pl = sh.plan[height - 1];
+    if (threadIdx.x >= 32) return;
+    if (threadIdx.x == 0) {
+        out[0] = pl.x;
+        out[1] = height;
+        out[2] = pl.y;
+        out[3] = pl.z;
+    }
+    for (int item = 0; item < min(pl.x, capacity); ++item) {
+        const WorkItem w = decode_item<kPrefix>(item, sh, work, host_plan, prefix, height);
+        if (threadIdx.x == 0) {
+            int *o = out + 4 + 8 * (int64_t)item;
+            o[0] = w.head;
+            o[1] = w.s0;
+            o[2] = w.s1;
+            o[3] = w.q_row0;
+            o[4] = w.q_hi;
+            o[5] = w.valid ? w.n_mt : 0;
+            o[6] = w.n_kv;
+            o[7] = 0;
+        }
+    }
+}
+
 // ---- host side --------------------------------------------------------------------------------------------------
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                   const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
@@ -1114,7 +1273,7 @@ bool attn_sm100_supported(const AttnArgs &a) {
 // and a failed attempt is retried by the next launch.
 template <typename Kernel> static int ensure_smem_optin(Kernel kernel, int slot, size_t smem) {
     static std::mutex mu;
-    static bool done[64][5];
+    static bool done[64][7];
     int dev = 0;
     COME_CUDA(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64) {
@@ -1132,34 +1291,31 @@ template <typename Kernel> static int ensure_smem_optin(Kernel kernel, int slot,
 static thread_local int t_cta_limit = 0;
 void attn_sm100_set_cta_limit(int max_ctas) { t_cta_limit = max_ctas > 0 ? max_ctas : 0; }
 
-int attn_sm100_launch(const AttnArgs &a, cudaStream_t stream) {
-    unsigned int *status = status_word_dev();
-    if (!status) return COME_ERR_CUDA;
-    CUtensorMap mq, mk, mv;
-    int rc;
-    if ((rc = make_map(&mq, a.q, a.dtype, a.q_end - a.q_begin, a.H, a.q_rs, kBlockM)) != COME_OK) return rc;
-    if ((rc = make_map(&mk, a.k, a.dtype, a.total, a.H, a.k_rs, kBlockN)) != COME_OK) return rc;
-    if ((rc = make_map(&mv, a.v, a.dtype, a.total, a.H, a.v_rs, kBlockN)) != COME_OK) return rc;
-    const bool with_table = !a.q_free && a.nseg >= kMinPrefixSegs && a.nseg <= kMaxPrefixSegs;
-    const size_t smem = sizeof(SharedStorage) + 1024 + (with_table ? kPrefixTableBytes : 0);
+struct LaunchPlan {
+    WorkPlan work;
+    bool with_table;
+    int span;       // most query rows a segment can own in this launch
+    unsigned grid;
+    int64_t items;  // upper bound; nothing to launch when it is 0
+};
+
+static int plan_launch(const AttnArgs &a, LaunchPlan *out) {
     const int64_t q_rows = a.q_end - a.q_begin;
     const int64_t span = a.q_free ? q_rows : (a.max_seqlen < q_rows ? a.max_seqlen : q_rows);  // most query rows any segment can own here
-    // Query tiles per work item: chosen on the device from the segments (0), except where the caller plans launches by
-    // their items (q_free: three tiles, see plan_tail_split) and where a launch has more segments than the table holds.
     int sms = sm_count();
     if (t_cta_limit > 0 && t_cta_limit < sms) sms = t_cta_limit;
+    // Query tiles per work item: chosen on the device from the segments (0) where there are several; on the host for one, for
+    // launches that give every query tile a CTA, where the caller plans launches by their items (q_free: three tiles, see
+    // plan_tail_split) and where a launch has more segments than the table holds.
     const int64_t most_tiles = (span + kBlockM - 1) / kBlockM;  // of one segment
-    int tiles = a.q_free ? 3 : a.nseg > kMaxPrefixSegs ? kTiles : 0;
-    if (tiles == 0 && most_tiles * a.nseg * a.H <= sms) {
-        tiles = 1;
-    } else if (tiles == 0 && a.nseg == 1 && a.max_seqlen_dev == nullptr) {
-        HeightSums hs = {};
-        hs.add((int)most_tiles);
-        tiles = hs.best(a.H, sms);
-    }
-    const int split_tail = !a.q_free && a.nseg <= kMaxPrefixSegs ? 1 : 0;  // launches whose items all exist
-    const int height = tiles == 0 || split_tail ? 1 : tiles;  // of the lowest items the launch may have
-    const int nblk_x = (int)((span + height * kBlockM - 1) / (height * kBlockM));
+    const bool with_table = !a.q_free && most_tiles > 1 && a.nseg >= kMinPrefixSegs && a.nseg <= kMaxPrefixSegs;
+    WorkPlan plan = {};
+    if (a.q_free) plan.height = 3;
+    else if (most_tiles == 1 || (!with_table && most_tiles * a.nseg * a.H <= sms)) plan.height = 1;
+    else if (a.nseg > kMaxPrefixSegs) plan.height = kTiles;
+    const bool one_segment = plan.height == 0 && a.nseg == 1 && a.max_seqlen_dev == nullptr;
+    const int height = plan.height == 0 ? 1 : plan.height;  // of the lowest items the launch may have
+    const int64_t nblk_x = (span + height * kBlockM - 1) / (height * kBlockM);
     const int k_parts = a.k_parts > 1 ? a.k_parts : 1;
     if (k_parts > 1) {
         // shares of the key tiles of every item: one segment whose keys all query rows attend to; no share may be empty
@@ -1170,23 +1326,68 @@ int attn_sm100_launch(const AttnArgs &a, cudaStream_t stream) {
             return COME_ERR_ARG;
         }
     }
-    const int64_t items = (int64_t)nblk_x * a.nseg * a.H * k_parts;
+    const int64_t items = nblk_x * a.nseg * a.H * k_parts;
+    out->items = items;
+    out->span = (int)span;
+    out->with_table = with_table;
     if (items <= 0) return COME_OK;
     if (items >= (1ll << 31)) {
         set_error("come_attn_varlen_fwd: %lld work items do not fit 32 bits", (long long)items);
         return COME_ERR_ARG;
     }
-    const unsigned grid = (unsigned)(items < sms ? items : sms);  // persistent: one CTA per SM walks the items
+    const unsigned grid = out->grid = (unsigned)(items < sms ? items : sms);  // persistent: one CTA per SM walks the items
+    if (one_segment) {
+        const int n = (int)most_tiles;
+        float least = 3.0e38f;
+        for (int h = kTiles; h >= 1; --h) {
+            WorkPlan p = {};
+            const int blocks = blocks_of(n, h), total = blocks * a.H, rest = total % (int)grid, rounds = total / (int)grid + (rest > 0 ? 1 : 0);
+            const float mean = (float)height_cost(n, h) / (float)blocks;
+            const float cost = split_last_round(p, h, total, rest, (float)rounds * mean, mean, 1.0f, (int)grid);
+            if (cost < least) {
+                least = cost;
+                plan = p;
+                plan.slots = blocks;
+            }
+        }
+    } else if (plan.height != 0) {
+        plan.slots = (int)nblk_x;
+        plan.total = plan.from = (int)items;
+        plan.parts = 1;
+    }
+    auto reciprocal = [](int64_t d) { return d > 0 ? (uint32_t)(0xffffffffu / (uint64_t)d) : 0u; };
+    plan.slots_rcp = reciprocal(plan.slots);
+    plan.nseg_rcp = reciprocal(a.nseg);
+    plan.ctas_rcp = reciprocal(grid);
+    out->work = plan;
+    return COME_OK;
+}
+
+int attn_sm100_launch(const AttnArgs &a, cudaStream_t stream) {
+    unsigned int *status = status_word_dev();
+    if (!status) return COME_ERR_CUDA;
+    CUtensorMap mq, mk, mv;
+    int rc;
+    if ((rc = make_map(&mq, a.q, a.dtype, a.q_end - a.q_begin, a.H, a.q_rs, kBlockM)) != COME_OK) return rc;
+    if ((rc = make_map(&mk, a.k, a.dtype, a.total, a.H, a.k_rs, kBlockN)) != COME_OK) return rc;
+    if ((rc = make_map(&mv, a.v, a.dtype, a.total, a.H, a.v_rs, kBlockN)) != COME_OK) return rc;
+    LaunchPlan plan;
+    if ((rc = plan_launch(a, &plan)) != COME_OK) return rc;
+    if (plan.items <= 0) return COME_OK;
+    const bool with_table = plan.with_table;
+    const unsigned grid = plan.grid;
+    const size_t smem = sizeof(SharedStorage) + 1024 + (with_table ? kPrefixTableBytes : 0);
+    const int k_parts = a.k_parts > 1 ? a.k_parts : 1;
     const float scale_log2 = a.scale * kLog2e;
     const float inv_scale = 1.0f / a.scale;
 #define COME_ATTN_LAUNCH(BF16, PREFIX, SELFTEST, SLOT)                                                                         \
     do {                                                                                                                       \
         if ((rc = ensure_smem_optin(attn_fwd_sm100_kernel<BF16, PREFIX, SELFTEST>, SLOT, smem)) != COME_OK) return rc;          \
         attn_fwd_sm100_kernel<BF16, PREFIX, SELFTEST><<<grid, kThreads, smem, stream>>>(mq, mk, mv, a.bias, a.cu, scale_log2, inv_scale, a.out, \
-                                                                              a.o_rs, a.lse, (int)a.q_begin, (int)a.q_end, tiles, (int)span, \
+                                                                              a.o_rs, a.lse, (int)a.q_begin, (int)a.q_end, plan.span, \
                                                                               a.nseg, a.H, a.max_seqlen_dev, status, (int)a.total,   \
-                                                                              a.q_free ? 1 : 0, split_tail, k_parts, (long long)a.part_o, \
-                                                                              (long long)a.part_l, a.stall_tile);                    \
+                                                                              a.q_free ? 1 : 0, k_parts, (long long)a.part_o, \
+                                                                              (long long)a.part_l, plan.work, a.stall_tile);         \
     } while (0)
     if (a.stall_tile >= 0) {
         COME_ATTN_LAUNCH(true, false, true, 4);
@@ -1238,4 +1439,36 @@ extern "C" int come_selftest_attn_stall(const void *qkv_dev, int64_t total, int 
     a.stall_tile = key_tiles;
     COME_REQUIRE(come::attn_sm100_supported(a), "come_selftest_attn_stall: needs 16-byte aligned tensors and a positive scale");
     return come::attn_sm100_launch(a, (cudaStream_t)stream);
+}
+
+extern "C" int come_attn_work_list(const int32_t *cu_seqlens_dev, int num_segments, int num_heads, int64_t q_row_begin, int64_t q_row_end,
+                                   int max_seqlen, const int32_t *max_seqlen_dev, int max_ctas, int32_t *out_dev, int64_t capacity, void *stream) {
+    COME_REQUIRE(cu_seqlens_dev && out_dev && num_segments > 0 && num_heads > 0 && max_seqlen > 0 && capacity >= 0 && capacity < (1ll << 28),
+                 "come_attn_work_list: bad arguments");
+    COME_REQUIRE(q_row_begin >= 0 && q_row_begin < q_row_end && q_row_end < (1ll << 31), "come_attn_work_list: bad row range");
+    using namespace come;
+    AttnArgs a = {};
+    a.q_begin = q_row_begin;
+    a.q_end = q_row_end;
+    a.H = num_heads;
+    a.nseg = num_segments;
+    a.max_seqlen = max_seqlen;
+    a.max_seqlen_dev = max_seqlen_dev;
+    LaunchPlan plan;
+    const int limit = t_cta_limit;
+    t_cta_limit = max_ctas;
+    int rc = plan_launch(a, &plan);
+    t_cta_limit = limit;
+    if (rc != COME_OK) return rc;
+    const size_t smem = sizeof(SharedStorage) + 1024 + kPrefixTableBytes;
+    if (plan.with_table) {
+        if ((rc = ensure_smem_optin(work_list_kernel<true>, 5, smem)) != COME_OK) return rc;
+        work_list_kernel<true><<<1, kThreads, smem, (cudaStream_t)stream>>>(cu_seqlens_dev, (int)q_row_begin, (int)q_row_end, plan.span, num_segments, num_heads,
+                                                                            max_seqlen_dev, (int)plan.grid, plan.work, out_dev, (int)capacity);
+    } else {
+        if ((rc = ensure_smem_optin(work_list_kernel<false>, 6, smem)) != COME_OK) return rc;
+        work_list_kernel<false><<<1, kThreads, smem, (cudaStream_t)stream>>>(cu_seqlens_dev, (int)q_row_begin, (int)q_row_end, plan.span, num_segments, num_heads,
+                                                                             max_seqlen_dev, (int)plan.grid, plan.work, out_dev, (int)capacity);
+    }
+    return check_launch("come_attn_work_list");
 }

@@ -385,6 +385,17 @@ int come_selftest_attn_stall(const void *qkv_dev, int64_t total, int num_heads, 
                              float softmax_scale, int key_tiles, void *out_dev, float *lse_dev, void *stream);
 
 /*
+ * The work list of a self-attention launch of the tensor-core kernel (head_dim 64) on at most max_ctas CTAs (0: one per SM),
+ * as the kernel forms it: for tests and for looking at the balance of a launch.  Arguments as in
+ * come_attn_varlen_fwd_rows.  out_dev receives items, query tiles per item, first item of a split last round, parts of a
+ * split item, and for each of the first `capacity` items 8 words: head, first key, last key + 1, first query row, end of the
+ * segment's query rows, 128-row query tiles (0: the item is skipped), 64-key tiles, tile slot of its first query tile.
+ */
+int come_attn_work_list(const int32_t *cu_seqlens_dev, int num_segments, int num_heads, int64_t q_row_begin, int64_t q_row_end,
+                        int max_seqlen, const int32_t *max_seqlen_dev, int max_ctas, int32_t *out_dev, int64_t capacity,
+                        void *stream);
+
+/*
  * Exchange of row blocks between the GPUs of one node through peer-mapped memory (one process per GPU): the transport of
  * the key / value all-gather of a global attention layer whose frames are sharded over the GPUs.  The reference has no
  * multi-GPU inference path; these entry points have no counterpart there.
