@@ -341,6 +341,7 @@ struct WorkItem {
     int head, s0, s1;   // head, key range of the segment
     int q_row0, q_hi;   // first query row of the item, end of the query rows this launch owns in the segment
     int n_mt, n_kv;     // active query tiles (1 .. kTiles), key tiles
+    int t0;             // tile slot of the first of them: items of one tile take the slots in turn, others begin at 0
     bool ragged_tail;   // the last key tile is partial
     bool valid;
     int kpart;          // which share of the keys this item covers (launches that split the keys of their items), else 0
@@ -602,6 +603,11 @@ __device__ __forceinline__ WorkItem decode_item(int item, const SharedStorage &s
                                                 int height) {
     WorkItem w;
     int bx, q_lo;
+    w.t0 = 0;
+    if (height == 1) {  // the round of the item
+        int cta;
+        w.t0 = div_by(item, a.ctas, host.ctas_rcp, cta) % kTiles;
+    }
     int first_tile = 0, most_tiles = height;  // of the item's rows inside its block of `height` tiles
     const int4 pl = sh.plan[height - 1];
     if (item >= pl.y) {
@@ -779,7 +785,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                     if (ok) {
                         mbar_arrive_expect_tx(&sh.q_full[b], w.n_mt * kQTileBytes);
                         for (int t = 0; t < w.n_mt; ++t)
-                            tma_load_3d(sh.q[b][t], &map_q, 0, w.head, w.q_row0 - q_begin + t * kBlockM, &sh.q_full[b]);
+                            tma_load_3d(sh.q[b][w.t0 + t], &map_q, 0, w.head, w.q_row0 - q_begin + t * kBlockM, &sh.q_full[b]);
                     }
                 }
                 ok = __all_sync(0xffffffffu, ok);
@@ -868,14 +874,15 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                         tc_mma_ts_1(o_tmem, p_tmem + 8 * i, vd + (uint64_t)(i * 128), idesc_pv, i > 0 ? 1u : accumulate);
                 };
                 struct Item {
-                    int n_mt, n_kv;
+                    uint32_t active;  // bit t: query tile t
+                    int n_kv;
                     bool ragged;
                 };
                 auto next_valid = [&](int &item, Item &x) -> bool {
                     for (; item < total_items; item += gridDim.x) {
                         const WorkItem w = decode_item<kPrefix>(item, sh, work, host_plan, prefix, height);
                         if (w.valid) {
-                            x = Item{w.n_mt, w.n_kv, w.ragged_tail};
+                            x = Item{((1u << w.n_mt) - 1u) << w.t0, w.n_kv, w.ragged_tail};
                             return true;
                         }
                     }
@@ -905,7 +912,8 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                     if (elect_one() && ok) {
 #pragma unroll
                         for (int t = first; t < kTiles; t += kIssuers)
-                            if (t < w.n_mt) qk(t, 0, 0, item_slab(w, 0));
+                            if ((w.active >> t) & 1u) qk(t, 0, 0, item_slab(w, 0));
+                        if (w.n_kv == 1) tc_commit_1(&sh.q_empty[0]);
                     }
                     __syncwarp();
                 }
@@ -922,7 +930,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                         const bool slab2 = item_slab(w, j + 1);
 #pragma unroll
                         for (int t = first; t < kTiles; t += kIssuers) {
-                            if (t < w.n_mt) {
+                            if ((w.active >> t) & 1u) {
                                 // O_t += P_t V, then the next scores of the tile over P_t: the tensor core executes them in order
                                 wait(sh.p_full[t], (p_phase >> t) & 1, kErrPFull);
                                 p_phase ^= 1u << t;
@@ -945,35 +953,36 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                     const uint32_t st2 = (st + 1) % kStages;
                     bool slab2 = false;
                     if (st2 == 0) kv_phase ^= 1u;
-                    if (have2) {
-                        wait(sh.kv_full[st2], kv_phase, kErrKvFull);
-                        wait(sh.q_full[qb ^ 1], (q_phase >> (qb ^ 1)) & 1, kErrQFull);
-                        q_phase ^= 1u << (qb ^ 1);
-                        slab2 = item_slab(nx, 0);
-                    } else {
-                        nx.n_mt = 0;
-                    }
+                    if (!have2) nx.active = 0;
+                    else slab2 = item_slab(nx, 0);
                     const uint32_t multi = w.n_kv > 1 ? 1u : 0u;
 #pragma unroll
                     for (int t = first; t < kTiles; t += kIssuers) {
-                        if (t < w.n_mt) {
+                        if ((w.active >> t) & 1u) {
                             wait(sh.p_full[t], (p_phase >> t) & 1, kErrPFull);
                             p_phase ^= 1u << t;
-                        }
-                        __syncwarp();
-                        tc_fence_after();
-                        if (elect_one() && ok) {
-                            if (t < w.n_mt) {
+                            __syncwarp();
+                            tc_fence_after();
+                            if (elect_one() && ok) {
                                 pv(t, st, multi);
                                 tc_commit_1(&sh.o_done[t]);
                             }
-                            if (t < nx.n_mt) qk(t, st2, qb ^ 1, slab2);
                         }
+                        __syncwarp();
+                        if (t == first && have2) {  // the next item's first loads: the P V in front needs none of them
+                            wait(sh.kv_full[st2], kv_phase, kErrKvFull);
+                            wait(sh.q_full[qb ^ 1], (q_phase >> (qb ^ 1)) & 1, kErrQFull);
+                            q_phase ^= 1u << (qb ^ 1);
+                            __syncwarp();
+                        }
+                        if (((nx.active >> t) & 1u) && elect_one() && ok) qk(t, st2, qb ^ 1, slab2);
                         __syncwarp();
                     }
                     if (elect_one() && ok) {
                         tc_commit_1(&sh.kv_empty[st]);
-                        tc_commit_1(&sh.q_empty[qb]);
+                        // Q is free behind the last scores; here with the last P V, except where an item is one key tile
+                        if (w.n_kv > 1) tc_commit_1(&sh.q_empty[qb]);
+                        if (have2 && nx.n_kv == 1) tc_commit_1(&sh.q_empty[qb ^ 1]);
                     }
                     __syncwarp();
                     st = st2;
@@ -1002,9 +1011,23 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         const uint32_t o_tmem = tmem + lane_addr + kTmemO + t * kHeadDim;
         bool ok = true;
         uint32_t s_phase = 0, o_phase = 0;
-        for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x) {
-            const WorkItem w = decode_item<kPrefix>(item, sh, work, host_plan, prefix, height);
-            if (!w.valid || t >= w.n_mt) continue;
+        struct Item {
+            int n_kv, row, q_hi, head, kpart;
+        };
+        auto next_active = [&](int &item, Item &x) -> bool {
+            for (; item < total_items; item += gridDim.x) {
+                const WorkItem w = decode_item<kPrefix>(item, sh, work, host_plan, prefix, height);
+                if (w.valid && (unsigned)(t - w.t0) < (unsigned)w.n_mt) {
+                    x = Item{w.n_kv, w.q_row0 + (t - w.t0) * kBlockM + r, w.q_hi, w.head, w.kpart};
+                    return true;
+                }
+            }
+            return false;
+        };
+        int item = blockIdx.x;
+        Item w;
+        bool have = next_active(item, w);
+        while (have && ok) {
             const int n_kv = w.n_kv;
             float m_ref = -INFINITY, l = 0.0f;  // reference max (log2 units, scale applied) and running sum
 
@@ -1077,6 +1100,14 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                 mbar_arrive(&sh.p_full[t]);
             }
 
+            // While the last P V runs: the next item, and what this one's epilogue needs beside the accumulator.
+            const bool in_range = w.row < w.q_hi;
+            const int64_t row = w.row - q_begin;
+            T *dst_row = reinterpret_cast<T *>(out_ptr) + (int64_t)w.kpart * part_o + row * o_rs + (int64_t)w.head * kHeadDim;
+            float *dst_lse = lse + (int64_t)w.kpart * part_l + (int64_t)w.head * (q_end - q_begin) + row;
+            item += gridDim.x;
+            have = next_active(item, w);
+            const float inv = 1.0f / l, row_lse = (m_ref + log2f(l)) * kLn2;
             if (ok) {
                 ok = mbar_wait(&sh.o_done[t], o_phase, sh, status, kErrODone);
                 o_phase ^= 1u;
@@ -1084,15 +1115,12 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
             }
             if (ok) {
                 tc_fence_after();
-                const int row = w.q_row0 + t * kBlockM + r;
-                const float inv = 1.0f / l;
-                T *dst_row = reinterpret_cast<T *>(out_ptr) + (int64_t)w.kpart * part_o + (int64_t)(row - q_begin) * o_rs + (int64_t)w.head * kHeadDim;
 #pragma unroll
                 for (int c = 0; c < 2; ++c) {
                     uint32_t o[32], pk[16];
                     tmem_ld32(o_tmem + 32 * c, o);
                     tc_wait_ld();  // the next item's first P V, which overwrites the accumulator, waits for this group's next P
-                    if (row < w.q_hi) {
+                    if (in_range) {
                         // The row's outputs as packed words, written with 32-byte stores where the address allows it: a warp's
                         // store then covers whole 32-byte sectors of its 32 rows instead of halves.
 #pragma unroll
@@ -1113,9 +1141,8 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                     }
                     __syncwarp();
                 }
+                if (lse && in_range) *dst_lse = row_lse;
                 tc_fence_before();  // the accumulator has been read; ordered before the next arrival on p_full
-                if (lse && row < w.q_hi)
-                    lse[(int64_t)w.kpart * part_l + (int64_t)w.head * (q_end - q_begin) + (row - q_begin)] = (m_ref + log2f(l)) * kLn2;
             }
         }
     }
@@ -1147,7 +1174,7 @@ __global__ void selftest_wait_kernel(long long ticks, unsigned int *__restrict__
 
 // The work list of a launch on `ctas` CTAs as the attention kernel walks it, for tests: out[0 .. 4) = items, query tiles per
 // item, first split item, parts of a split one; then per item head, first and last + 1 key, first query row, end of the query
-// rows, query tiles (0: skipped), key tiles
+// rows, query tiles (0: skipped), key tiles, first tile slot.
 template <bool kPrefix>
 __global__ void __launch_bounds__(kThreads, 1)
 work_list_kernel(const int *__restrict__ cu, int q_begin, int q_end, int max_rows, int nseg, int num_heads, const int *__restrict__ max_len_dev, int ctas,
@@ -1179,7 +1206,7 @@ work_list_kernel(const int *__restrict__ cu, int q_begin, int q_end, int max_row
             o[4] = w.q_hi;
             o[5] = w.valid ? w.n_mt : 0;
             o[6] = w.n_kv;
-            o[7] = 0;
+            o[7] = w.t0;
         }
     }
 }

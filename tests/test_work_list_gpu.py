@@ -84,7 +84,7 @@ def _check(lengths, heads, ctas, rows=None, bound=None, device_bound=None):
         assert max(s0, span[0]) <= row < end == min(s1, span[1])
         low = height if i < split else (1 if parts == height else 2)
         assert 1 <= tiles <= low
-        assert slot == 0
+        assert slot == ((i // ctas) % 4 if height == 1 else 0) and slot + tiles <= 4
         seen[head, row - span[0]: min(end, row + tiles * TILE) - span[0]] += 1
     assert (seen == 1).all()
     table = 16 <= len(lengths) <= 2048 and most > 1
