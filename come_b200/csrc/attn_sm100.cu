@@ -39,6 +39,7 @@
 
 #include <cuda.h>
 
+#include <algorithm>
 #include <mutex>
 #include <type_traits>
 
@@ -1353,7 +1354,9 @@ static int plan_launch(const AttnArgs &a, LaunchPlan *out) {
             return COME_ERR_ARG;
         }
     }
-    const int64_t items = nblk_x * a.nseg * a.H * k_parts;
+    // an exact list holds no more than the rows' tiles and a partial one per segment, however loose max_seqlen is
+    const int64_t slots = nblk_x * a.nseg, blocks = plan.height == 0 ? std::min(slots, q_rows / kBlockM + a.nseg) : slots;
+    const int64_t items = blocks * a.H * k_parts, slot_items = slots * a.H * k_parts;
     out->items = items;
     out->span = (int)span;
     out->with_table = with_table;
@@ -1362,7 +1365,7 @@ static int plan_launch(const AttnArgs &a, LaunchPlan *out) {
         set_error("come_attn_varlen_fwd: %lld work items do not fit 32 bits", (long long)items);
         return COME_ERR_ARG;
     }
-    const unsigned grid = out->grid = (unsigned)(items < sms ? items : sms);  // persistent: one CTA per SM walks the items
+    const unsigned grid = out->grid = (unsigned)(slot_items < sms ? slot_items : sms);  // persistent: one CTA per SM walks the items
     if (one_segment) {
         const int n = (int)most_tiles;
         float least = 3.0e38f;

@@ -124,6 +124,18 @@ def test_row_slices_and_device_bounds():
     _check([1374], 4, 5, bound=2748, device_bound=1374)
 
 
+def test_loose_bound_does_not_count():
+    """2048 segments of 8192 tokens x 16 heads are 2 million items; with the sum of all lengths as the bound of the longest one
+    2^32 slots could exist, which no launch holds."""
+    from come_b200 import _lib
+    from come_b200._torch_util import ptr, stream_ptr
+    cu = torch.arange(0, 2049, dtype=torch.int32, device="cuda") * 8192
+    total = 2048 * 8192
+    out = torch.zeros(4 + 8, dtype=torch.int32, device="cuda")
+    _lib.check(_lib.lib().come_attn_work_list(ptr(cu), 2048, 16, 0, total, total, None, 0, ptr(out), 1, stream_ptr(cu.device)))
+    assert out[1].item() == 4 and 2048 * 16 * 16 <= out[0].item() < 2048 * 16 * 16 + 4 * 148
+
+
 def test_all_heights_and_splits_are_reached():
     """The lengths of the attention tests that compare bits over the number of CTAs take every height and every split."""
     reached = set()
