@@ -265,7 +265,7 @@ def cross_fwd(q_rows, k, v, perkey_bias, softmax_scale, out_=None):
     return [out, lse]
 
 
-_ROWS_PER_ITEM = 384  # query rows of a work item of the tensor-core kernel (three 128-row tiles)
+_ROWS_PER_ITEM = 384  # query rows of a work item of a cross launch (three 128-row tiles; other launches take one to four)
 
 
 def plan_tail_split(rows: int, num_heads: int, kv_rows: int, ctas: int):

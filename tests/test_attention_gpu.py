@@ -243,9 +243,9 @@ def test_query_row_slices_match_full_attention(backend, which, seq_lens, cuts):
 
 
 def test_tile_boundary_lengths(backend):
-    """Segment lengths on and around the kernel's tile sizes (64 keys per step, 128-row query tiles, 384-row work items):
-    every combination of one, two or three active query tiles and of a full or ragged last key tile, and more work items
-    than SMs so that CTAs of the persistent kernel carry their barrier phases across several items."""
+    """Segment lengths on and around the kernel's tile sizes (64 keys per step, 128-row query tiles, work items of up to four
+    of them): one to four active query tiles with a full or ragged last key tile, and more work items than SMs so that CTAs
+    of the persistent kernel carry their barrier phases across several items."""
     from come_b200 import flash_attn as api, flash_attn_fwd_cuda as fa
     backend(fa.BACKEND_TCGEN05)
     rng = np.random.default_rng(12)
@@ -287,8 +287,8 @@ def test_device_side_longest_segment(backend):
 @pytest.mark.parametrize("lengths", [[897], [1, 128, 129, 256, 257, 384, 385, 511, 512, 513], [60 + 31 * i for i in range(17)]])
 def test_item_heights(backend, kind, lengths):
     """The kernel picks one to four query tiles per work item from the segments and the number of CTAs (on the host for one
-    segment, on the device without and with the per-segment table).  Every number of CTAs gives the same bits, whatever the
-    height, and the oracle's values."""
+    segment, on the device without and with the per-segment table; test_work_list_gpu.py shows that these lengths and numbers
+    of CTAs take all four heights).  Every number of CTAs gives the same bits, whatever the height, and the oracle's values."""
     from come_b200 import flash_attn_fwd_cuda as fa
     backend(fa.BACKEND_TCGEN05)
     rng = np.random.default_rng(len(lengths))
